@@ -6,8 +6,9 @@
 //
 // One cluster of CTAs, barriers between its phases in hardware.  Bound by the latency of those phases: a row is
 // 0.3 MB.  A row of 151 936 bf16 logits (top-k 20, top-p 0.95) takes 59 us where one logit stands out and 305 us where none
-// does, f32 89 and 338; on one CTA that added term by term, 1.2, 12.3, 1.7 and 29 ms.  With filters the row is sorted for real (stable LSD radix sort, 8-bit digits), because the reference's
-// cut depends on f32 sums accumulated one after another in that order.  The sums keep the bits of that chain
+// does, f32 89 and 338; on one CTA that added term by term, 1.2, 12.3, 1.7 and 29 ms.  With filters the row is sorted
+// for real (stable LSD radix sort, 8-bit digits), because the reference's cut depends on f32 sums accumulated one after
+// another in that order.  The sums keep the bits of that chain
 // without running it: between two powers of two every addition moves the sum by a whole number of its units in the
 // last place, which depends on the sum only through its parity where a term lies half way between two of them, so
 // stretches of terms compose (sum_in_order).
@@ -16,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "cluster_fit.cuh"
 #include "context.cuh"
 #include "ops.cuh"
 
@@ -646,26 +648,16 @@ stark_b200_status sampling_launch(const void *logits, uint32_t io_type, uint32_t
     p.idx[0] = base + 2u * (size_t)vocab;
     p.idx[1] = base + 4u * (size_t)vocab;  // with the array behind it: the ordered sampler's f64 terms, 8-byte aligned
     p.out = out_device;
-    // 16 CTAs where the device can hold such a cluster (it takes more than the portable 8)
-    static const uint32_t cluster = [] {
-        uint32_t fits = 16u;
-        for (const void *f : {(const void *)unified_sampling_kernel, (const void *)ordered_sampling_kernel}) {
-            if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) fits = 8u;
-            cudaLaunchConfig_t c = sampling_config(fits, nullptr);
-            cudaLaunchAttribute a = cluster_of(fits);
-            c.attrs = &a;
-            c.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, f, &c) != cudaSuccess || n < 1) fits = 8u;
-        }
-        cudaGetLastError();
-        return fits;
-    }();
+    const bool ordered = (s.flags & 32u) != 0;
+    static ClusterFit known[2];
+    const auto kernel = ordered ? ordered_sampling_kernel : unified_sampling_kernel;
+    const uint32_t cluster = cluster_fit((const void *)kernel, sampling_config(0u, stream), known[ordered]);
+    if (!cluster) return STARK_B200_DEVICE_FAILURE;
     cudaLaunchConfig_t config = sampling_config(cluster, stream);
     cudaLaunchAttribute attribute = cluster_of(cluster);
     config.attrs = &attribute;
     config.numAttrs = 1;
-    SB_CUDA(cudaLaunchKernelEx(&config, (s.flags & 32u) ? ordered_sampling_kernel : unified_sampling_kernel, p));
+    SB_CUDA(cudaLaunchKernelEx(&config, kernel, p));
     return STARK_B200_OK;
 }
 

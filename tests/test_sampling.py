@@ -1,6 +1,9 @@
 """The stochastic sampler: the oracle against the published Philox4x32-10 known answers and the
 reference's own unit-interval test, host-side seed derivation, and (GPU) the device sampler against
 the oracle on seeded rows."""
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -125,6 +128,60 @@ def test_device_sampler_on_awkward_rows(kind, vocab):
             total += 1
     # a near-tie of noisy scores can resolve differently under the device's expf / logf, in both forms of the row
     assert agree >= total - 2, (agree, total)
+
+
+CLUSTER_FIT = """
+#include "cluster_fit.cuh"
+#include <cstdio>
+using namespace sb;
+// A runtime of three devices: 0 and 2 hold clusters of 16 of a kernel opted in there, 1 does not.
+static int current = 0, opted[3][2], queries = 0, errors = 0;
+static int kernels[2];
+static int which(const void *f) { return f == &kernels[1]; }
+extern "C" cudaError_t cudaGetDevice(int *d) { *d = current; return cudaSuccess; }
+extern "C" cudaError_t cudaGetLastError() { ++errors; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v) {
+    opted[current][which(f)] += a == cudaFuncAttributeNonPortableClusterSizeAllowed && v == 1;
+    return cudaSuccess;
+}
+extern "C" cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *f, const cudaLaunchConfig_t *c) {
+    ++queries;
+    *n = current != 1 && opted[current][which(f)] && c->gridDim.x == 16 && c->numAttrs == 1 && c->attrs->val.clusterDim.x == 16;
+    return current == 1 ? cudaErrorInvalidClusterSize : cudaSuccess;
+}
+int main() {
+    static ClusterFit known[2];
+    for (int round = 0; round < 2; ++round)
+        for (current = 0; current < 3; ++current)
+            for (int k = 0; k < 2; ++k) std::printf("%u ", cluster_fit(&kernels[k], cudaLaunchConfig_t{}, known[k]));
+    std::printf("| %d %d %d %d %d", queries, errors, opted[0][0], opted[1][1], opted[2][0]);
+}
+"""
+
+
+def test_cluster_size_is_known_per_device(tmp_path):
+    """What one device allows says nothing about another: every device is opted in and asked once, for each kernel."""
+    src, exe = tmp_path / "fit.cpp", tmp_path / "fit"
+    src.write_text(CLUSTER_FIT)
+    root = Path(__file__).resolve().parents[1]
+    subprocess.run(["g++", "-std=c++17", f"-I{root / 'stark_b200' / 'csrc'}", "-I/usr/local/cuda/include", str(src), "-o", str(exe)],
+                   check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    assert out == "16 16 8 8 16 16 " * 2 + "| 6 2 1 1 1", out
+
+
+@pytest.mark.gpu
+def test_sampler_on_two_devices():
+    from stark_b200 import _lib, ops
+    if ops.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    row = np.random.default_rng(4).standard_normal(9000).astype(np.float32)
+    for ordered in (False, True):
+        seen = []
+        for device in (0, 1, 0):
+            _lib.check(_lib.load().stark_b200_set_device(device), "set_device")
+            seen.append(ops.sample(row, seed=11, temperature=0.8, top_k=40, ordered=ordered))
+        assert len(set(seen)) == 1
 
 
 @pytest.mark.gpu
