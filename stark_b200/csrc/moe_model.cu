@@ -964,7 +964,7 @@ size_t moe_rows_carve(const stark_b200_moe_config &c, uint32_t rows, uint8_t *ba
 bool moe_rows_ready(const MoeModel *m) {
     const auto &c = m->cfg;
     const uint32_t group = c.q_heads / c.kv_heads, widest = std::max(std::max(c.hidden, c.q_heads * c.head_dim), c.expert_intermediate);
-    if (m->ep.ranks > 1u || (group != 8u && group != 4u && group != 2u) || widest > 12288u) return false;
+    if (m->ep.ranks > 1u || (group != 8u && group != 4u && group != 2u) || widest > kMoeRowsWidest) return false;
     for (uint32_t l = 0; l < c.layers; ++l)
         if (m->qkv[l]->format != kFmtQ8_0T || m->o[l]->format != kFmtQ8_0T || m->gate_up[l]->format != kFmtQ4_K ||
             m->down[l]->format != kFmtQ4_K)

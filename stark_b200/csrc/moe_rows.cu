@@ -519,6 +519,15 @@ stark_b200_status launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_
     return STARK_B200_OK;
 }
 
+// The kernels that hold a row in shared memory: the widest takes 48 KB beside their own words, more than a launch has unasked.
+template <typename... Params, typename... Args>
+stark_b200_status launch_row(SmemOptIn &once, void (*kernel)(Params...), dim3 grid, dim3 block, uint32_t columns, cudaStream_t stream,
+                             Args... args) {
+    if (columns > kMoeRowsWidest) return STARK_B200_UNSUPPORTED;
+    if (stark_b200_status s = ensure_dynamic_smem(kernel, (int)kMoeRowsWidest * 4, once)) return s;
+    return launch(kernel, grid, block, (size_t)columns * 4u, stream, args...);
+}
+
 constexpr size_t gemm_smem(uint32_t stages, uint32_t warps, uint32_t super_bytes, uint32_t sums) {
     return stages * (warps * super_bytes + kTileLines * kLine + sums);
 }
@@ -577,7 +586,8 @@ stark_b200_status rows_q4k_experts_launch(const QMatrix *w, uint32_t blocks, con
 
 stark_b200_status moe_rows_embed_launch(const uint32_t *tokens, const uint8_t *table, float *x, const float *w, float eps,
                                         const RowsOperand &out, uint32_t rows, cudaStream_t stream) {
-    return launch(moe_rows_embed_kernel, rows, kRowThreads, (size_t)out.columns * 4u, stream, tokens, table, x, w, eps, out);
+    static SmemOptIn once;
+    return launch_row(once, moe_rows_embed_kernel, rows, kRowThreads, out.columns, stream, tokens, table, x, w, eps, out);
 }
 
 stark_b200_status moe_rows_heads_launch(float *qkv, const float *q_norm, const float *k_norm, float *keys, float *values,
@@ -590,13 +600,15 @@ stark_b200_status moe_rows_heads_launch(float *qkv, const float *q_norm, const f
 stark_b200_status moe_rows_merge_launch(const float *part, uint32_t heads, uint32_t splits, const RowsOperand &out,
                                         uint32_t rows, cudaStream_t stream) {
     if (out.columns != heads * 128u) return STARK_B200_INVALID_ARGUMENT;
-    return launch(moe_rows_merge_kernel, rows, kRowThreads, (size_t)out.columns * 4u, stream, part, splits, out);
+    static SmemOptIn once;
+    return launch_row(once, moe_rows_merge_kernel, rows, kRowThreads, out.columns, stream, part, splits, out);
 }
 
 stark_b200_status moe_rows_add_norm_launch(float *x, const float *update, const float *probs, uint32_t active, const float *w,
                                            float eps, float *normed, const RowsOperand &out, uint32_t rows, uint32_t hidden,
                                            cudaStream_t stream) {
-    return launch(moe_rows_add_norm_kernel, rows, kRowThreads, (size_t)hidden * 4u, stream, x, update, probs, active, w, eps,
+    static SmemOptIn once;
+    return launch_row(once, moe_rows_add_norm_kernel, rows, kRowThreads, hidden, stream, x, update, probs, active, w, eps,
                   normed, out, hidden);
 }
 
@@ -617,7 +629,8 @@ stark_b200_status moe_rows_lists_launch(const MoeRowLists &lists, uint32_t rows,
 
 stark_b200_status moe_rows_gate_launch(const float *gate_up, uint32_t inter, const RowsOperand &out, uint32_t pairs,
                                        cudaStream_t stream) {
-    return launch(moe_rows_gate_kernel, pairs, kGateThreads, (size_t)inter * 4u, stream, gate_up, out);
+    static SmemOptIn once;
+    return launch_row(once, moe_rows_gate_kernel, pairs, kGateThreads, inter, stream, gate_up, out);
 }
 
 }  // namespace sb

@@ -5,6 +5,7 @@
 namespace sb {
 
 constexpr uint32_t kMoeRowsMax = 512;    // rows of one pass
+constexpr uint32_t kMoeRowsWidest = 12288;  // columns of the widest row
 constexpr uint32_t kMoeRowsChunk = 16;   // rows that share one reading of a weight record
 
 // Input rows of a contraction: every row as f16 head and f16 remainder of row * 2^s (s by the row's largest element),

@@ -225,6 +225,32 @@ def test_prompt_rows_in_passes(name, portions):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [
+    dict(hidden=12288), dict(hidden=12544), dict(q_heads=96, kv_heads=12), dict(q_heads=98, kv_heads=49), dict(inter=12288), dict(inter=12544)])
+def test_prompt_rows_of_the_widest_models(sizes):
+    """Row widths at the most that a pass of rows takes and one step past it: rows go one by one then, and input rows of q, k, v
+    and o past the matvec's own bound are refused."""
+    from stark_b200._lib import StarkB200Error
+    from stark_b200.engine import MoEModel
+    cfg = dict(S.MOE_CONFIGS["moe-tiny"], layers=2, experts=4, active=2, **sizes)
+    w = S.moe_weights(cfg, seed=12)
+    model, oracle = MoEModel.load(cfg, w, 24), O.MoEDecoder(cfg, w, 24)
+    ids = S.prompt(cfg, 19, seed=2)
+    if max(cfg["hidden"], 128 * cfg["q_heads"]) > 12288:
+        for call in (lambda: model.ingest(ids[:1]), lambda: model.ingest(ids[:-1])):
+            with pytest.raises(StarkB200Error, match="unsupported"):
+                call()
+        model.close()
+        return
+    model.ingest(ids[:-1])
+    oracle.ingest(ids[:-1])
+    assert model.position == 18
+    assert model.last_experts().tolist() == oracle.last_experts.tolist()
+    assert _close(model.step(int(ids[-1])), oracle.step(int(ids[-1])))
+    model.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("sizes,behind", [
     (dict(hidden=4608, inter=4352, experts=4, active=3, q_heads=2, kv_heads=1), 0),    # rows of more super-blocks than warps
     (dict(hidden=256, inter=256, experts=300, active=32, q_heads=8, kv_heads=2), 15),  # one warp a row tile; most picks
