@@ -130,7 +130,7 @@ __global__ void moe_heads_kernel(const MoeState *st, float *qkv, const float *q_
         return;
     }
     const float v = src[i];
-    float s = v * v;
+    float s = __fmul_rn(v, v);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((i & 31u) == 0) scratch[i >> 5] = s;
@@ -138,14 +138,14 @@ __global__ void moe_heads_kernel(const MoeState *st, float *qkv, const float *q_
     float sum = 0.0f;
     for (uint32_t w = 0; w < dim / 32u; ++w) sum += scratch[w];
     const float scale = 1.0f / sqrtf(sum / (float)dim + eps);
-    head[i] = v * scale * (h < q_heads ? q_norm : k_norm)[i];
+    head[i] = __fmul_rn(__fmul_rn(v, scale), (h < q_heads ? q_norm : k_norm)[i]);
     __syncthreads();
     const uint32_t half = dim / 2u, pair = i < half ? i : i - half;
-    const float angle = (float)position * powf(theta, -((float)(2u * pair)) / (float)dim);
+    const float angle = __fmul_rn((float)position, powf(theta, -((float)(2u * pair)) / (float)dim));
     float sn, cs;
     sincosf(angle, &sn, &cs);
     const float a = head[pair], b = head[pair + half];
-    const float out = i < half ? a * cs - b * sn : a * sn + b * cs;
+    const float out = i < half ? fmaf(a, cs, -__fmul_rn(b, sn)) : fmaf(a, sn, __fmul_rn(b, cs));  // prepare_head's bits
     if (h < q_heads)
         src[i] = out;
     else
@@ -231,26 +231,22 @@ __global__ void __launch_bounds__(kAttnWarps * 32) moe_attention_kernel(const Mo
 // The same attention with the query heads of one KV head handled together (G = q_heads / kv_heads): a CTA
 // per (KV head, span) reads each K and V row once and scores it against all G queries, instead of G CTAs
 // reading the same rows.  Per warp: G running (max, sum, accumulator) states; warp g merges head g's states.
-// gridDim.z > 1: that many rows from the state's position on, `q_row` apart in q.
 template <int G>
 __global__ void __launch_bounds__(kAttnWarps * 32) moe_attention_grouped_kernel(const MoeState *st, const float *q,
                                                                                 const float *keys, const float *values, float *part,
                                                                                 uint32_t splits, uint32_t kv_heads,
-                                                                                float scale, uint32_t context,
-                                                                                uint32_t q_row) {
+                                                                                float scale, uint32_t context) {
     constexpr uint32_t D = 128;
     __shared__ float sm[kAttnWarps][G], sl[kAttnWarps][G];
     __shared__ float4 sacc[kAttnWarps][G][32];
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t kvh = blockIdx.x, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t rows = min(st->position + 1u + blockIdx.z, context);
+    const uint32_t rows = min(st->position + 1u, context);
     const uint32_t span = (rows + splits - 1u) / splits;
     const uint32_t lo = min(rows, split * span), hi = min(rows, lo + span);
     const size_t kv_row = (size_t)kv_heads * D;
     const uint32_t begin = kvh * D;
-    q += (size_t)blockIdx.z * q_row;
-    part += (size_t)blockIdx.z * kv_heads * G * splits * (D + 2u);
     float4 qv[G];
 #pragma unroll
     for (int g = 0; g < G; ++g)
@@ -521,7 +517,7 @@ __global__ void __launch_bounds__(1024) moe_ep_mix_norm_kernel(float *x, const u
             }
 #pragma unroll
             for (uint32_t j = 0; j < 8u; ++j)
-                if (e0 + j < active) r += sp[e0 + j] * __uint_as_float((uint32_t)q[j]);
+                if (e0 + j < active) r = fmaf(sp[e0 + j], __uint_as_float((uint32_t)q[j]), r);  // token_mix_kernel's bits
         }
         const float v = x[i] + r;
         x[i] = v;
@@ -716,22 +712,6 @@ struct MoeModel {
 
 namespace {
 
-template <typename... Params, typename... Args>
-stark_b200_status moe_launch(void (*kernel)(Params...), dim3 grid, dim3 block, bool pdl, cudaStream_t stream,
-                             Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    SB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
-    return STARK_B200_OK;
-}
-
 // Every kernel of a token awaits its predecessor itself (programmatic dependent launch), so the next
 // kernel's CTAs are placed, and the matvecs' first weight records fetched, while the previous one drains.
 // STARK_B200_PDL=0 serializes the launches instead.
@@ -743,7 +723,7 @@ bool moe_pdl() {
     return on;
 }
 
-// CTAs of the grouped attention kernel over all KV heads (STARK_B200_MOE_ATTN_CTAS overrides).
+// CTAs of a token's attention over all KV heads (STARK_B200_MOE_ATTN_CTAS overrides).
 uint32_t moe_attention_ctas() {
     static const uint32_t n = [] {
         const char *e = getenv("STARK_B200_MOE_ATTN_CTAS");
@@ -753,6 +733,10 @@ uint32_t moe_attention_ctas() {
     return n;
 }
 
+uint32_t moe_splits(const stark_b200_moe_config &c) {
+    return std::max(kAttnSplits, std::min(kMoeMaxAttnSplits, moe_attention_ctas() / c.kv_heads));
+}
+
 // A token whose matrices, head groups or row lengths the kernels of moe_token.cu do not take; n holds the normed row at its end.
 stark_b200_status moe_issue_general(MoeModel *m, bool want_logits, cudaStream_t s) {
     const auto &c = m->cfg;
@@ -760,16 +744,16 @@ stark_b200_status moe_issue_general(MoeModel *m, bool want_logits, cudaStream_t 
     const uint32_t I = c.expert_intermediate;
     const float scale = 1.0f / sqrtf((float)D);
     const bool pdl = moe_pdl();
-    SB_TRY(moe_launch(moe_rmsnorm_kernel, 1, 1024, pdl, s, m->x, m->norm(STARK_B200_MOE_TENSOR_ATTN_NORM, 0), m->n, H,
+    SB_TRY(moe_launch(moe_rmsnorm_kernel, 1, 1024, 0, pdl, s, m->x, m->norm(STARK_B200_MOE_TENSOR_ATTN_NORM, 0), m->n, H,
                       c.rms_eps));
     for (uint32_t l = 0; l < c.layers; ++l) {
         float *keys = m->keys + (size_t)l * m->kv_layer(), *values = m->values + (size_t)l * m->kv_layer();
         uint32_t *ids = m->ids + (size_t)l * 2u * A;
         SB_TRY(qmv_rows_launch(m->qkv[l], m->n, 0, m->qkv_out, 1, nullptr, STARK_B200_F32, s, pdl));
         // query heads of one KV head together where the group size has an instantiation, else head by head
-        const uint32_t group = QH / KV, gsplits = std::max(kAttnSplits, std::min(kMoeMaxAttnSplits, moe_attention_ctas() / KV));
+        const uint32_t group = QH / KV, gsplits = moe_splits(c);
         const bool grouped_form = group == 8u || group == 4u || group == 2u;
-        SB_TRY(moe_launch(moe_heads_kernel, QH + 2u * KV, D, pdl, s, m->state, m->qkv_out,
+        SB_TRY(moe_launch(moe_heads_kernel, QH + 2u * KV, D, 0, pdl, s, m->state, m->qkv_out,
                           m->norm(STARK_B200_MOE_TENSOR_Q_NORM, l), m->norm(STARK_B200_MOE_TENSOR_K_NORM, l), keys, values, QH, KV,
                           D, c.rms_eps, c.rope_theta, c.context_tokens));
         uint32_t splits = kAttnSplits;
@@ -777,18 +761,18 @@ stark_b200_status moe_issue_general(MoeModel *m, bool want_logits, cudaStream_t 
             splits = gsplits;
             auto grouped = group == 8u ? moe_attention_grouped_kernel<8>
                                        : (group == 4u ? moe_attention_grouped_kernel<4> : moe_attention_grouped_kernel<2>);
-            SB_TRY(moe_launch(grouped, dim3(KV, splits), kAttnWarps * 32, pdl, s, m->state, m->qkv_out, keys, values,
-                              m->part, splits, KV, scale, c.context_tokens, 0u));
+            SB_TRY(moe_launch(grouped, dim3(KV, splits), kAttnWarps * 32, 0, pdl, s, m->state, m->qkv_out, keys, values,
+                              m->part, splits, KV, scale, c.context_tokens));
         } else {
-            SB_TRY(moe_launch(moe_attention_kernel, dim3(QH, kAttnSplits), kAttnWarps * 32, pdl, s, m->state, m->qkv_out,
+            SB_TRY(moe_launch(moe_attention_kernel, dim3(QH, kAttnSplits), kAttnWarps * 32, 0, pdl, s, m->state, m->qkv_out,
                               keys, values, m->part, QH, KV, scale, c.context_tokens));
         }
-        SB_TRY(moe_launch(moe_attention_merge_kernel, QH, 128, pdl, s, m->part, m->att, splits));
+        SB_TRY(moe_launch(moe_attention_merge_kernel, QH, 128, 0, pdl, s, m->part, m->att, splits));
         SB_TRY(qmv_rows_launch(m->o[l], m->att, 0, m->update, 1, nullptr, STARK_B200_F32, s, pdl));
-        SB_TRY(moe_launch(moe_add_norm_kernel, 1, 1024, pdl, s, m->x, m->update, nullptr, 1u,
+        SB_TRY(moe_launch(moe_add_norm_kernel, 1, 1024, 0, pdl, s, m->x, m->update, nullptr, 1u,
                           m->norm(STARK_B200_MOE_TENSOR_FFN_NORM, l), m->n, H, c.rms_eps));
         const bool ep = m->ep.ranks > 1u;
-        SB_TRY(moe_launch(moe_router_select_kernel, c.experts, 256, pdl, s, m->router + (size_t)l * c.experts * H, m->n,
+        SB_TRY(moe_launch(moe_router_select_kernel, c.experts, 256, 0, pdl, s, m->router + (size_t)l * c.experts * H, m->n,
                           m->scores, H, c.experts, A, ids, m->probs, m->arrivals,
                           ep ? m->ids_global + (size_t)l * A : nullptr, ep ? m->ep.rank * m->ep.local_experts : 0u,
                           ep ? m->ep.local_experts : 0u));
@@ -797,7 +781,7 @@ stark_b200_status moe_issue_general(MoeModel *m, bool want_logits, cudaStream_t 
             SB_TRY(q4kt_launch(m->down[l], m->gate_out, I, m->expert_out, A, ids, STARK_B200_F32, s, pdl,
                                m->gate_out + (size_t)A * I));
         } else {
-            SB_TRY(moe_launch(moe_silu_mul_kernel, (A * I + 255u) / 256u, 256, pdl, s, m->gate_out,
+            SB_TRY(moe_launch(moe_silu_mul_kernel, (A * I + 255u) / 256u, 256, 0, pdl, s, m->gate_out,
                               m->gate_out + (size_t)A * I, A * I));
             SB_TRY(qmv_rows_launch(m->down[l], m->gate_out, I, m->expert_out, A, ids, STARK_B200_F32, s, pdl));
         }
@@ -805,11 +789,11 @@ stark_b200_status moe_issue_general(MoeModel *m, bool want_logits, cudaStream_t 
         const float *next = l + 1u < c.layers ? m->norm(STARK_B200_MOE_TENSOR_ATTN_NORM, l + 1u)
                                               : (want_logits ? m->norm(STARK_B200_MOE_TENSOR_FINAL_NORM, 0) : nullptr);
         if (ep) {
-            SB_TRY(moe_launch(moe_ep_push_kernel, A, 256, pdl, s, m->ep, m->expert_out, ids, l, c.layers, A, H, m->ep_tokens));
-            SB_TRY(moe_launch(moe_ep_mix_norm_kernel, 1, 1024, pdl, s, m->x, ep_packets(m->ep_local, l, A, H), m->probs, A,
+            SB_TRY(moe_launch(moe_ep_push_kernel, A, 256, 0, pdl, s, m->ep, m->expert_out, ids, l, c.layers, A, H, m->ep_tokens));
+            SB_TRY(moe_launch(moe_ep_mix_norm_kernel, 1, 1024, 0, pdl, s, m->x, ep_packets(m->ep_local, l, A, H), m->probs, A,
                               next, m->n, H, c.rms_eps, m->ep_tokens, l, c.layers, m->ep.wait_ns, m->state));
         } else {
-            SB_TRY(moe_launch(moe_add_norm_kernel, 1, 1024, pdl, s, m->x, m->expert_out, m->probs, A, next, m->n, H,
+            SB_TRY(moe_launch(moe_add_norm_kernel, 1, 1024, 0, pdl, s, m->x, m->expert_out, m->probs, A, next, m->n, H,
                               c.rms_eps));
         }
     }
@@ -833,7 +817,7 @@ bool moe_fused(const MoeModel *m) { return (m->fuse < 0 ? m->ep.ranks <= 1u : m-
 stark_b200_status moe_issue_tiled(MoeModel *m, bool want_logits, cudaStream_t s) {
     const auto &c = m->cfg;
     const uint32_t H = c.hidden, D = c.head_dim, QH = c.q_heads, KV = c.kv_heads, A = c.active_experts;
-    const uint32_t splits = std::max(kAttnSplits, std::min(kMoeMaxAttnSplits, moe_attention_ctas() / KV));
+    const uint32_t splits = moe_splits(c);
     const bool pdl = moe_pdl(), fused = moe_fused(m), ep = m->ep.ranks > 1u;
     const uint32_t *position = &m->state->position;
     for (uint32_t l = 0; l < c.layers; ++l) {
@@ -843,7 +827,7 @@ stark_b200_status moe_issue_tiled(MoeModel *m, bool want_logits, cudaStream_t s)
         const float *q_norm = m->norm(STARK_B200_MOE_TENSOR_Q_NORM, l), *k_norm = m->norm(STARK_B200_MOE_TENSOR_K_NORM, l);
         SB_TRY(token_q8_launch(m->qkv[l], m->x, attn_norm, c.rms_eps, nullptr, m->qkv_out, pdl, s));
         if (!fused)
-            SB_TRY(moe_launch(moe_heads_kernel, QH + 2u * KV, D, pdl, s, m->state, m->qkv_out, q_norm, k_norm, keys, values, QH, KV,
+            SB_TRY(moe_launch(moe_heads_kernel, QH + 2u * KV, D, 0, pdl, s, m->state, m->qkv_out, q_norm, k_norm, keys, values, QH, KV,
                               D, c.rms_eps, c.rope_theta, c.context_tokens));
         SB_TRY(token_attention_launch(position, m->qkv_out, fused, keys, values, m->part, splits, QH, KV, c.context_tokens, q_norm,
                                       k_norm, c.rms_eps, c.rope_theta, pdl, s));
@@ -856,15 +840,15 @@ stark_b200_status moe_issue_tiled(MoeModel *m, bool want_logits, cudaStream_t s)
         SB_TRY(token_gate_up_launch(m->gate_up[l], sel, m->x, ffn_norm, c.rms_eps, m->gate_out, pdl, s));
         SB_TRY(token_down_launch(m->down[l], ids, A, m->gate_out, m->expert_out, pdl, s));
         if (ep) {
-            SB_TRY(moe_launch(moe_ep_push_kernel, A, 256, pdl, s, m->ep, m->expert_out, ids, l, c.layers, A, H, m->ep_tokens));
-            SB_TRY(moe_launch(moe_ep_mix_norm_kernel, 1, 1024, pdl, s, m->x, ep_packets(m->ep_local, l, A, H), m->probs, A, nullptr,
+            SB_TRY(moe_launch(moe_ep_push_kernel, A, 256, 0, pdl, s, m->ep, m->expert_out, ids, l, c.layers, A, H, m->ep_tokens));
+            SB_TRY(moe_launch(moe_ep_mix_norm_kernel, 1, 1024, 0, pdl, s, m->x, ep_packets(m->ep_local, l, A, H), m->probs, A, nullptr,
                               m->n, H, c.rms_eps, m->ep_tokens, l, c.layers, m->ep.wait_ns, m->state));
         } else {
             SB_TRY(token_mix_launch(m->x, m->expert_out, m->probs, A, H, pdl, s));
         }
     }
     if (want_logits)
-        SB_TRY(moe_launch(moe_rmsnorm_kernel, 1, 1024, pdl, s, m->x, m->norm(STARK_B200_MOE_TENSOR_FINAL_NORM, 0), m->n, H,
+        SB_TRY(moe_launch(moe_rmsnorm_kernel, 1, 1024, 0, pdl, s, m->x, m->norm(STARK_B200_MOE_TENSOR_FINAL_NORM, 0), m->n, H,
                           c.rms_eps));
     return STARK_B200_OK;
 }
@@ -872,13 +856,13 @@ stark_b200_status moe_issue_tiled(MoeModel *m, bool want_logits, cudaStream_t s)
 stark_b200_status moe_issue(MoeModel *m, bool want_logits, cudaStream_t s) {
     const auto &c = m->cfg;
     const bool pdl = moe_pdl();
-    SB_TRY(moe_launch(moe_embed_kernel, 1, 256, false, s, m->state, m->token_table, m->x, c.hidden, c.vocab, c.context_tokens));
+    SB_TRY(moe_launch(moe_embed_kernel, 1, 256, 0, false, s, m->state, m->token_table, m->x, c.hidden, c.vocab, c.context_tokens));
     SB_TRY(moe_tiled(m) ? moe_issue_tiled(m, want_logits, s) : moe_issue_general(m, want_logits, s));
     if (want_logits) SB_TRY(qmv_rows_launch(m->output, m->n, 0, m->logits, 1, nullptr, STARK_B200_F32, s, pdl));
     // the attention partials are free by now: scratch for the per-CTA maxima
-    SB_TRY(moe_launch(moe_finish_kernel, want_logits ? kFinishCtas : 1u, 1024, pdl, s, m->state,
+    SB_TRY(moe_launch(moe_finish_kernel, want_logits ? kFinishCtas : 1u, 1024, 0, pdl, s, m->state,
                       want_logits ? m->logits : nullptr, c.vocab, m->part, m->arrivals + 1));
-    if (m->ep.ranks > 1u) SB_TRY(moe_launch(moe_ep_token_barrier_kernel, 1, 32, false, s, m->ep, m->ep_tokens, m->state));
+    if (m->ep.ranks > 1u) SB_TRY(moe_launch(moe_ep_token_barrier_kernel, 1, 32, 0, false, s, m->ep, m->ep_tokens, m->state));
     return STARK_B200_OK;
 }
 
@@ -919,17 +903,14 @@ stark_b200_status moe_token(MoeModel *m, bool want_logits) {
 
 // Working memory of a prompt pass, carved out of one allocation.
 struct MoeRowsWork {
-    float *x, *normed, *qkv, *update, *gate_up, *expert_out, *part;
+    float *x, *qkv, *update, *gate_up, *expert_out, *part;
+    size_t part_floats;
     uint32_t *tokens;
     RowsOperand hidden, attended, gated;
     MoeRowLists lists;
 };
 
-// CTAs of the attention of a pass over all rows and KV heads: few rows over a long cache divide it among more of them, 32 keys
-// at least (11 rows at the start of the cache: the merge of 16 spans, most of them empty, took 67 us of a layer's 270).
-uint32_t rows_attention_splits(const stark_b200_moe_config &c, uint32_t rows, uint32_t keys) {
-    return std::max(1u, std::min(kAttnSplits, std::min(1024u / (rows * c.kv_heads), keys / 32u)));
-}
+constexpr size_t kMoePartFloats = (size_t)16 << 20;  // states of the spans of the rows that attend at once: half of L2
 
 size_t moe_rows_carve(const stark_b200_moe_config &c, uint32_t rows, uint8_t *base, MoeRowsWork *w) {
     const size_t H = c.hidden, QD = (size_t)c.q_heads * c.head_dim, KD = (size_t)c.kv_heads * c.head_dim;
@@ -942,71 +923,57 @@ size_t moe_rows_carve(const stark_b200_moe_config &c, uint32_t rows, uint8_t *ba
     };
     const auto floats = [&](size_t n) { return reinterpret_cast<float *>(take(n * 4u)); };
     const auto words = [&](size_t n) { return reinterpret_cast<uint32_t *>(take(n * 4u)); };
-    const auto operand = [&](RowsOperand &o, size_t n, size_t columns) {
+    const auto operand = [&](RowsOperand &o, size_t n, size_t columns, bool norm) {
         o.split = reinterpret_cast<__half *>(take(n * columns * 4u));
-        o.unscale = floats(n);
-        o.sums = floats(n * (columns / 32u));
+        o.meta = floats(n * (columns / kSlice) * kRowsMeta);
+        o.scale = norm ? floats(n) : nullptr;
         o.columns = (uint32_t)columns;
     };
-    size_t part = 0;  // fewer rows take more spans each
-    for (uint32_t r = 1; r <= rows; ++r) part = std::max(part, (size_t)r * c.q_heads * rows_attention_splits(c, r, c.context_tokens) * (c.head_dim + 2u));
-    w->x = floats(R * H), w->normed = floats(R * H), w->qkv = floats(R * (QD + 2u * KD)), w->update = floats(R * H);
-    w->gate_up = floats(R * A * 2u * I), w->expert_out = floats(R * A * H), w->part = floats(part);
+    const size_t row_part = moe_rows_part(c.q_heads, moe_rows_spans(moe_splits(c), c.context_tokens));
+    w->part_floats = std::min(R * row_part, std::max(kMoePartFloats, row_part));
+    w->x = floats(R * H), w->qkv = floats(R * (QD + 2u * KD)), w->update = floats(R * H);
+    w->gate_up = floats(R * A * 2u * I), w->expert_out = floats(R * A * H), w->part = floats(w->part_floats);
     w->tokens = words(R);
-    operand(w->hidden, R, H), operand(w->attended, R, QD), operand(w->gated, R * A, I);
+    operand(w->hidden, R, H, true), operand(w->attended, R, QD, false), operand(w->gated, R * A, I, false);
     w->lists.ids = words(R * A), w->lists.probs = floats(R * A), w->lists.scores = floats(R * c.experts), w->lists.pairs = words(R * A);
     w->lists.tiles = words(1u + 3u * MoeRowLists::max_tiles(rows, c.active_experts, c.experts));
     return at;
 }
 
-// Whether prompt rows of this model can run in passes: one GPU, re-tiled matrices, a group size the attention kernel has, rows
-// that fit the pass's shared memory.  Everything else is ingested token by token.
-bool moe_rows_ready(const MoeModel *m) {
-    const auto &c = m->cfg;
-    const uint32_t group = c.q_heads / c.kv_heads, widest = std::max(std::max(c.hidden, c.q_heads * c.head_dim), c.expert_intermediate);
-    if (m->ep.ranks > 1u || (group != 8u && group != 4u && group != 2u) || widest > kMoeRowsWidest) return false;
-    for (uint32_t l = 0; l < c.layers; ++l)
-        if (m->qkv[l]->format != kFmtQ8_0T || m->o[l]->format != kFmtQ8_0T || m->gate_up[l]->format != kFmtQ4_K ||
-            m->down[l]->format != kFmtQ4_K)
-            return false;
-    return true;
-}
+// Whether prompt rows of this model can run in passes: one GPU, and tokens that take the kernels whose sums a pass forms.
+// Everything else is ingested token by token.
+bool moe_rows_ready(const MoeModel *m) { return m->ep.ranks <= 1u && moe_tiled(m); }
 
-// `rows` prompt rows at the model's position, cache only: the operators of moe_issue over all rows at once.  What follows the
-// last layer's expert selection reaches neither the cache nor last_experts and is not run.
+// `rows` prompt rows at the model's position, cache only: the operators of moe_issue_tiled over all rows at once, to the bit.
+// What follows the last layer's expert selection reaches neither the cache nor last_experts and is not run.
 stark_b200_status moe_rows_pass(MoeModel *m, const uint32_t *tokens, uint32_t rows) {
     const auto &c = m->cfg;
-    const uint32_t H = c.hidden, D = c.head_dim, QH = c.q_heads, KV = c.kv_heads, A = c.active_experts, I = c.expert_intermediate;
+    const uint32_t H = c.hidden, QH = c.q_heads, KV = c.kv_heads, A = c.active_experts;
     const cudaStream_t s = m->stream;
     MoeRowsWork w{};
     moe_rows_carve(c, m->rows_capacity, m->rows_work, &w);
     SB_CUDA(cudaMemcpyAsync(w.tokens, tokens, (size_t)rows * 4u, cudaMemcpyHostToDevice, s));
     SB_TRY(moe_rows_embed_launch(w.tokens, m->token_table, w.x, m->norm(STARK_B200_MOE_TENSOR_ATTN_NORM, 0), c.rms_eps, w.hidden,
                                  rows, s));
-    const uint32_t splits = rows_attention_splits(c, rows, m->position + rows), group = QH / KV, q_row = (QH + 2u * KV) * D;
-    const auto attention = group == 8u ? moe_attention_grouped_kernel<8>
-                                       : (group == 4u ? moe_attention_grouped_kernel<4> : moe_attention_grouped_kernel<2>);
     for (uint32_t l = 0; l < c.layers; ++l) {
         float *keys = m->keys + (size_t)l * m->kv_layer(), *values = m->values + (size_t)l * m->kv_layer();
-        const bool last = l + 1u == c.layers;
+        const float *ffn_norm = m->norm(STARK_B200_MOE_TENSOR_FFN_NORM, l);
         SB_TRY(rows_q8_launch(m->qkv[l], w.hidden, w.qkv, rows, s));
         SB_TRY(moe_rows_heads_launch(w.qkv, m->norm(STARK_B200_MOE_TENSOR_Q_NORM, l), m->norm(STARK_B200_MOE_TENSOR_K_NORM, l),
-                                     keys, values, QH, KV, D, c.rms_eps, c.rope_theta, m->position, rows, s));
-        SB_TRY(moe_launch(attention, dim3(KV, splits, rows), kAttnWarps * 32, true, s, m->state, w.qkv, keys, values, w.part,
-                          splits, KV, 1.0f / sqrtf((float)D), c.context_tokens, q_row));
-        SB_TRY(moe_rows_merge_launch(w.part, QH, splits, w.attended, rows, s));
+                                     keys, values, QH, KV, c.rms_eps, c.rope_theta, m->position, rows, s));
+        SB_TRY(moe_rows_attention_launch(w.qkv, keys, values, w.part, w.part_floats, QH, KV, moe_splits(c), m->position, w.attended,
+                                         rows, s));
         SB_TRY(rows_q8_launch(m->o[l], w.attended, w.update, rows, s));
-        SB_TRY(moe_rows_add_norm_launch(w.x, w.update, nullptr, 0, m->norm(STARK_B200_MOE_TENSOR_FFN_NORM, l), c.rms_eps, w.normed,
-                                        w.hidden, rows, H, s));
-        SB_TRY(moe_rows_route_launch(m->router + (size_t)l * c.experts * H, w.normed, H, c.experts, A, w.lists,
+        SB_TRY(moe_rows_add_norm_launch(w.x, w.update, nullptr, 0, ffn_norm, c.rms_eps, w.hidden, rows, s));
+        SB_TRY(moe_rows_route_launch(m->router + (size_t)l * c.experts * H, w.x, ffn_norm, w.hidden, c.experts, A, w.lists,
                                      m->ids + (size_t)l * 2u * A, rows, s));
-        if (last) break;
+        if (l + 1u == c.layers) break;
         SB_TRY(moe_rows_lists_launch(w.lists, rows, A, c.experts, s));
         SB_TRY(rows_q4k_experts_launch(m->gate_up[l], 2u, w.hidden, A, w.gate_up, w.lists, rows, A, s));
-        SB_TRY(moe_rows_gate_launch(w.gate_up, I, w.gated, rows * A, s));
+        SB_TRY(moe_rows_gate_launch(w.gate_up, w.gated, rows * A, s));
         SB_TRY(rows_q4k_experts_launch(m->down[l], 1u, w.gated, 1u, w.expert_out, w.lists, rows, A, s));
-        SB_TRY(moe_rows_add_norm_launch(w.x, w.expert_out, w.lists.probs, A, m->norm(STARK_B200_MOE_TENSOR_ATTN_NORM, l + 1u),
-                                        c.rms_eps, nullptr, w.hidden, rows, H, s));
+        SB_TRY(moe_rows_add_norm_launch(w.x, w.expert_out, w.lists.probs, A, m->norm(STARK_B200_MOE_TENSOR_ATTN_NORM, l + 1u), c.rms_eps,
+                                        w.hidden, rows, s));
     }
     m->position += rows;
     SB_CUDA(cudaMemcpyAsync(&m->state->position, &m->position, 4u, cudaMemcpyHostToDevice, s));

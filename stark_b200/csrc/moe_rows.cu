@@ -1,4 +1,4 @@
-// Prompt rows of the routed-expert decoder: a pass of up to 512 rows through the operators of a token (moe_model.cu), f32
+// Prompt rows of the routed-expert decoder: a pass of up to 512 rows through the operators of a token (moe_token.cu), f32
 // activations throughout.  The reference batches them in 256-row passes with the rows grouped by expert
 // (crates/stark-engine/src/encodable_block/decoder.rs:182-186, mlp/routed.rs:144-256).
 //
@@ -8,13 +8,13 @@
 // applied in f32 to every sub-block's sums.  (tcgen05 accumulates over the whole contraction, so the scales would have to
 // go into the weights, which then need a remainder of their own and the input's 22 bits three products instead of two.)
 //
-// 12 layers of the 30B-A3B shape, 160 rows and the token behind them: 5.9 ms against 112 ms token by token.
+// Every sum over a row, a slice of 256 columns, a strand of keys or the spans is formed as a token forms it (moe_math.cuh): a
+// row's results are the token's, bit for bit.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
 
 #include "context.cuh"
-#include "gguf_math.cuh"
 #include "moe_rows.cuh"
 #include "moe_select.cuh"
 
@@ -26,13 +26,16 @@ constexpr uint32_t kNt = kMoeRowsChunk / 4u;         // column tiles of four row
 static_assert(kNt == 4u, "run() below has a loop for each");
 constexpr uint32_t kLine = 512u + 64u;               // a row's head or remainder of 256 columns: two lines 64 B apart modulo 128 B
 constexpr uint32_t kTileLines = kMoeRowsChunk * 2u;  // lines of a stage
+template <bool Q4>
+constexpr uint32_t kMetaBytes = Q4 ? kRowsMeta * 4u : 16u;  // of a row's slice: the scale; the sums behind it
 
 struct RowsGemmParams {
     const uint8_t *data;
-    uint32_t rows, row_tiles, supers, row_blocks;  // of one matrix; row_blocks: its CTAs
+    uint32_t rows, row_tiles, row_blocks;  // of one matrix; row_blocks: its CTAs
+    Members at;
     size_t matrix_bytes;
     const __half *x;
-    const float *unscale, *sums;
+    const float *meta, *scale;
     float *out;
     uint32_t out_stride;
     uint32_t m;                            // dense: input rows
@@ -40,13 +43,23 @@ struct RowsGemmParams {
     uint32_t divisor, experts;
 };
 
+// The slices in the order in which a token adds them up: member by member.  `ends`: the member's last.
+__device__ inline uint32_t slice_at(const Members &at, uint32_t step, bool &ends) {
+    const uint32_t full = at.supers - (at.records - 1u) * at.width;  // members with `records` slices, the first ones
+    const bool late = step >= full * at.records;
+    const uint32_t each = at.records - (late ? 1u : 0u), k = late ? step - full * at.records : step;
+    ends = k % each + 1u == each;
+    return (late ? full : 0u) + k / each + k % each * at.width;
+}
+
 // One CTA: 16 matrix rows a warp times up to 16 input rows, the contraction in steps of 256 columns, copies of the
 // next steps in flight.  Bound by issue slots of the tensor-core loop at full tiles (10 instructions per two products) and by
 // the weights' bytes where experts have few rows.
-template <bool Q4, int STAGES, uint32_t WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8u ? 2 : 1) rows_gemm_kernel(const RowsGemmParams p) {
-    constexpr uint32_t kSuper = Q4 ? kQ4SuperBytes : kB8SuperBytes;
-    constexpr uint32_t kStage = WARPS * kSuper + kTileLines * kLine + (Q4 ? kMoeRowsChunk * 32u : 0u);
+// MULTI: members of several slices.
+template <bool Q4, int STAGES, uint32_t WARPS, bool MULTI>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8u && !MULTI ? 2 : 1) rows_gemm_kernel(const RowsGemmParams p) {
+    constexpr uint32_t kSuper = Q4 ? kQ4SuperBytes : kB8SuperBytes, kMeta = kMetaBytes<Q4>;
+    constexpr uint32_t kStage = WARPS * kSuper + kTileLines * kLine + kMoeRowsChunk * kMeta;
     extern __shared__ __align__(16) uint8_t rows_smem[];
     __shared__ uint32_t ids[kMoeRowsChunk];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t = lane & 3u;
@@ -66,15 +79,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8u ? 2 : 1) rows_gemm_ker
         if (tid < count) ids[tid] = first + tid;
     }
     __syncthreads();
-    const uint32_t row_tile = block * WARPS + warp;
+    const uint32_t row_tile = block * WARPS + warp, supers = p.at.supers;
     const bool live = row_tile < p.row_tiles;
-    const uint8_t *weights = p.data + (size_t)matrix * p.matrix_bytes + (size_t)row_tile * p.supers * kSuper;
-    const size_t columns = (size_t)p.supers * 256u;
+    const uint8_t *weights = p.data + (size_t)matrix * p.matrix_bytes + (size_t)row_tile * supers * kSuper;
+    const size_t columns = (size_t)supers * kSlice;
     const uint32_t live_nt = (count + 3u) / 4u;
 
-    const auto issue = [&](uint32_t s) {
-        if (s < p.supers) {
-            uint8_t *stage = rows_smem + (s % STAGES) * kStage;
+    const auto issue = [&](uint32_t step) {
+        if (step < supers) {
+            bool ends;
+            const uint32_t s = MULTI ? slice_at(p.at, step, ends) : step;
+            uint8_t *stage = rows_smem + (step % STAGES) * kStage;
             if (live)
                 for (uint32_t off = lane * 16u; off < kSuper; off += 512u)
                     cp_async16(stage + warp * kSuper + off, weights + (size_t)s * kSuper + off);
@@ -82,78 +97,112 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8u ? 2 : 1) rows_gemm_ker
             for (uint32_t i = tid; i < count * 64u; i += WARPS * 32u) {
                 const uint32_t line = i >> 5, c = i & 31u;
                 cp_async16(lines + line * kLine + c * 16u,
-                           p.x + ((size_t)(ids[line >> 1] / p.divisor) * 2u + (line & 1u)) * columns + s * 256u + c * 8u);
+                           p.x + ((size_t)(ids[line >> 1] / p.divisor) * 2u + (line & 1u)) * columns + s * kSlice + c * 8u);
             }
-            if (Q4 && tid < count * 2u)
-                cp_async16(lines + kTileLines * kLine + tid * 16u,
-                           p.sums + (size_t)(ids[tid >> 1] / p.divisor) * (p.supers * 8u) + s * 8u + (tid & 1u) * 4u);
+            constexpr uint32_t kChunks = kMeta / 16u;
+            for (uint32_t i = tid; i < count * kChunks; i += WARPS * 32u)
+                cp_async16(lines + kTileLines * kLine + i * 16u,
+                           p.meta + ((size_t)(ids[i / kChunks] / p.divisor) * supers + s) * kRowsMeta + i % kChunks * 4u);
         }
         cp_async_commit();
     };
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) issue(s);
 
-    float acc0[kNt], acc1[kNt];  // matrix rows g and g + 8, input row t of every column tile
+    float acc0[kNt], acc1[kNt], part0[kNt], part1[kNt];  // matrix rows g and g + 8, input row t of every column tile; of a member
 #pragma unroll
-    for (uint32_t n = 0; n < kNt; ++n) acc0[n] = acc1[n] = 0.0f;
+    for (uint32_t n = 0; n < kNt; ++n) acc0[n] = acc1[n] = part0[n] = part1[n] = 0.0f;
     // The loop for a number of column tiles known to the compiler: their products are independent chains, which a test in
     // between kept apart (a warp waited 2.6 cycles an instruction for the one before it).
     const auto run = [&](auto tiles) {
         constexpr uint32_t NT = decltype(tiles)::value;
-        for (uint32_t s = 0; s < p.supers; ++s) {
+        for (uint32_t step = 0; step < supers; ++step) {
             cp_async_wait<STAGES - 2>();
             __syncthreads();  // every thread's copies of this step are there, and everybody is done with the step before
-            issue(s + STAGES - 1);
+            issue(step + STAGES - 1);
             if (!live) continue;
-            const uint8_t *rec = rows_smem + (s % STAGES) * kStage + warp * kSuper;
-            const uint8_t *lines = rows_smem + (s % STAGES) * kStage + WARPS * kSuper + g * kLine + t * 16u;
-            const float *sums = reinterpret_cast<const float *>(rows_smem + (s % STAGES) * kStage + WARPS * kSuper + kTileLines * kLine);
+            const uint8_t *stage = rows_smem + (step % STAGES) * kStage, *rec = stage + warp * kSuper;
+            const uint8_t *lines = stage + WARPS * kSuper + g * kLine + t * 16u;
+            const uint8_t *meta = stage + WARPS * kSuper + kTileLines * kLine + t * kMeta;  // of input row t; 4 kMeta to the next tile's
             float dsc0[2], dm0[2], dsc1[2], dm1[2];
             if (Q4) {
                 q4k_scales_pair(*reinterpret_cast<const uint4 *>(rec + 2048u + 16u * g), t, dsc0, dm0);
                 q4k_scales_pair(*reinterpret_cast<const uint4 *>(rec + 2048u + 16u * (g + 8u)), t, dsc1, dm1);
             }
+            // What sub-blocks q and q + 4 add: the share of lane q of a token's row.
+            const auto shares = [&](uint32_t q, float(&r0)[NT], float(&r1)[NT]) {
 #pragma unroll
-            for (uint32_t jb = 0; jb < 8; ++jb) {
-                uint32_t a[8];
-                float s0, s1, m0 = 0.0f, m1 = 0.0f;
-                if (Q4) {
-                    const uint2 w = *reinterpret_cast<const uint2 *>(rec + jb * 256u + lane * 8u);
-                    dequant_a4_word<0>(w.x, *reinterpret_cast<uint32_t(*)[4]>(&a[0]));
-                    dequant_a4_word<0>(w.y, *reinterpret_cast<uint32_t(*)[4]>(&a[4]));
-                    // lane jb mod 4 of the four that share these rows decoded this sub-block's scales
-                    const uint32_t from = (lane & ~3u) | (jb & 3u);
-                    s0 = __shfl_sync(0xffffffffu, dsc0[jb >> 2], from), s1 = __shfl_sync(0xffffffffu, dsc1[jb >> 2], from);
-                    m0 = __shfl_sync(0xffffffffu, dm0[jb >> 2], from), m1 = __shfl_sync(0xffffffffu, dm1[jb >> 2], from);
-                } else {
-                    const uint4 w = *reinterpret_cast<const uint4 *>(rec + jb * 512u + lane * 16u);
-                    bytes_to_f16<false>(w.x, a[0], a[1]);
-                    bytes_to_f16<false>(w.y, a[2], a[3]);
-                    bytes_to_f16<false>(w.z, a[4], a[5]);
-                    bytes_to_f16<false>(w.w, a[6], a[7]);
-                    const uint16_t *meta = reinterpret_cast<const uint16_t *>(rec + 4096u);
-                    s0 = f16_bits_f32(meta[jb * 16u + g]), s1 = f16_bits_f32(meta[jb * 16u + g + 8u]);
-                }
-                uint4 xv[NT];
-                float c[NT][4];
-#pragma unroll
-                for (uint32_t n = 0; n < NT; ++n) {
-                    xv[n] = *reinterpret_cast<const uint4 *>(lines + n * 8u * kLine + jb * 64u);
-                    c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.0f;
-                }
-#pragma unroll
-                for (uint32_t n = 0; n < NT; ++n) mma_m16n8k16_f16(c[n], *reinterpret_cast<uint32_t(*)[4]>(&a[0]), xv[n].x, xv[n].y);
-#pragma unroll
-                for (uint32_t n = 0; n < NT; ++n) mma_m16n8k16_f16(c[n], *reinterpret_cast<uint32_t(*)[4]>(&a[4]), xv[n].z, xv[n].w);
-#pragma unroll
-                for (uint32_t n = 0; n < NT; ++n) {
-                    acc0[n] = fmaf(s0, c[n][0] + c[n][1], acc0[n]);
-                    acc1[n] = fmaf(s1, c[n][2] + c[n][3], acc1[n]);
+                for (int h = 1; h >= 0; --h) {
+                    const uint32_t jb = q + 4u * h;
+                    uint32_t a[8];
                     if (Q4) {
-                        const float xs = sums[(n * 4u + t) * 8u + jb];
-                        acc0[n] = fmaf(-m0, xs, acc0[n]);
-                        acc1[n] = fmaf(-m1, xs, acc1[n]);
+                        const uint2 w = *reinterpret_cast<const uint2 *>(rec + jb * 256u + lane * 8u);
+                        dequant_a4_word<0>(w.x, *reinterpret_cast<uint32_t(*)[4]>(&a[0]));
+                        dequant_a4_word<0>(w.y, *reinterpret_cast<uint32_t(*)[4]>(&a[4]));
+                    } else {
+                        const uint4 w = *reinterpret_cast<const uint4 *>(rec + jb * 512u + lane * 16u);
+                        bytes_to_f16<false>(w.x, a[0], a[1]);
+                        bytes_to_f16<false>(w.y, a[2], a[3]);
+                        bytes_to_f16<false>(w.z, a[4], a[5]);
+                        bytes_to_f16<false>(w.w, a[6], a[7]);
                     }
+                    uint4 xv[NT];
+                    float c[NT][4];
+#pragma unroll
+                    for (uint32_t n = 0; n < NT; ++n) {
+                        xv[n] = *reinterpret_cast<const uint4 *>(lines + n * 8u * kLine + jb * 64u);
+                        c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.0f;
+                    }
+#pragma unroll
+                    for (uint32_t n = 0; n < NT; ++n) mma_m16n8k16_f16(c[n], *reinterpret_cast<uint32_t(*)[4]>(&a[0]), xv[n].x, xv[n].y);
+#pragma unroll
+                    for (uint32_t n = 0; n < NT; ++n) mma_m16n8k16_f16(c[n], *reinterpret_cast<uint32_t(*)[4]>(&a[4]), xv[n].z, xv[n].w);
+                    float s0, s1, m0 = 0.0f, m1 = 0.0f, n0 = 0.0f, n1 = 0.0f;
+                    if (Q4) {  // lane q of the four that share these rows decoded these sub-blocks' scales
+                        const uint32_t from = (lane & ~3u) | q;
+                        s0 = __shfl_sync(0xffffffffu, dsc0[h], from), s1 = __shfl_sync(0xffffffffu, dsc1[h], from);
+                        if (h == 1) {
+                            m0 = __shfl_sync(0xffffffffu, dm0[0], from), m1 = __shfl_sync(0xffffffffu, dm1[0], from);
+                            n0 = __shfl_sync(0xffffffffu, dm0[1], from), n1 = __shfl_sync(0xffffffffu, dm1[1], from);
+                        }
+                    } else {
+                        const uint16_t *scales = reinterpret_cast<const uint16_t *>(rec + 4096u) + jb * 16u + g;
+                        s0 = f16_bits_f32(scales[0]), s1 = f16_bits_f32(scales[8]);
+                    }
+#pragma unroll
+                    for (uint32_t n = 0; n < NT; ++n) {
+                        const float p0 = c[n][0] + c[n][1], p1 = c[n][2] + c[n][3];
+                        if (h == 0) {
+                            r0[n] = share_first(s0, p0, r0[n]), r1[n] = share_first(s1, p1, r1[n]);
+                        } else if (Q4) {
+                            const float *sums = reinterpret_cast<const float *>(meta + 4u * n * kMeta) + 4u + q;
+                            r0[n] = q4k_share_second(s0, p0, m0, sums[0], n0, sums[4]);
+                            r1[n] = q4k_share_second(s1, p1, m1, sums[0], n1, sums[4]);
+                        } else {
+                            r0[n] = q8_share_second(s0, p0), r1[n] = q8_share_second(s1, p1);
+                        }
+                    }
+                }
+            };
+            float sum0[NT] = {}, sum1[NT] = {};
+#pragma unroll 1  // two shares at a time: four in one stretch spill
+            for (uint32_t q = 0; q < 4u; q += 2u) {
+                float a0[NT], a1[NT], b0[NT], b1[NT];
+                shares(q, a0, a1);
+                shares(q + 1u, b0, b1);
+#pragma unroll
+                for (uint32_t n = 0; n < NT; ++n) sum0[n] += a0[n] + b0[n], sum1[n] += a1[n] + b1[n];
+            }
+            bool ends = true;
+            if (MULTI) slice_at(p.at, step, ends);
+#pragma unroll
+            for (uint32_t n = 0; n < NT; ++n) {
+                const float down = *reinterpret_cast<const float *>(meta + 4u * n * kMeta);
+                if (MULTI) {
+                    part0[n] = fmaf(down, sum0[n], part0[n]), part1[n] = fmaf(down, sum1[n], part1[n]);
+                    if (ends) acc0[n] += part0[n], acc1[n] += part1[n], part0[n] = part1[n] = 0.0f;
+                } else {
+                    acc0[n] = __fadd_rn(acc0[n], __fmul_rn(down, sum0[n])), acc1[n] = __fadd_rn(acc1[n], __fmul_rn(down, sum1[n]));
                 }
             }
         }
@@ -170,244 +219,304 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8u ? 2 : 1) rows_gemm_ker
         const uint32_t i = n * 4u + t;
         if (i >= count) continue;
         const uint32_t id = ids[i];
-        const float unscale = p.unscale[id / p.divisor];
+        const float scale = p.scale ? p.scale[id / p.divisor] : 1.0f;
         float *y = p.out + (size_t)id * p.out_stride + column;
-        if (r0 < p.rows) y[r0] = acc0[n] * unscale;
-        if (r1 < p.rows) y[r1] = acc1[n] * unscale;
+        if (r0 < p.rows) y[r0] = __fmul_rn(acc0[n], scale);
+        if (r1 < p.rows) y[r1] = __fmul_rn(acc1[n], scale);
     }
 }
 
-template <int THREADS, typename F>
-__device__ inline float row_reduce(float v, F f, float *scratch /* [THREADS / 32] */) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, o));
+// A slice of an operand row, by one warp.
+__device__ inline void store_slice(const RowsOperand &out, uint32_t at, uint32_t s, const float (&v)[8]) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const SplitSlice split = split_slice(v);
+    __half *head = out.split + (size_t)at * 2u * out.columns + s * kSlice + lane * 8u;
+    *reinterpret_cast<uint4 *>(head) = split.head;
+    *reinterpret_cast<uint4 *>(head + out.columns) = split.rest;
+    float *meta = out.meta + ((size_t)at * (out.columns / kSlice) + s) * kRowsMeta;
+    if ((lane & 3u) == 0) meta[4u + lane / 4u] = split.sum;
+    if (lane == 0) meta[0] = split.down;
+}
+
+// rms_norm(row, w) as an operand, a warp a member of the row: `value` gives a lane's eight columns of a slice.
+template <typename Value>
+__device__ inline void norm_operand(const RowsOperand &out, uint32_t at, const Members &members, const float *w, float eps, Value value) {
+    __shared__ float squares[kMaxMembers];
+    const uint32_t lane = threadIdx.x & 31u, member = threadIdx.x >> 5;
+    float square = 0.0f;
+    for (uint32_t s = member; s < members.supers; s += members.width) {
+        float v[8], g[8];
+        load8(w + s * kSlice + lane * 8u, g);
+        value(s, v);
+        weigh8(v, g, square);
+        store_slice(out, at, s, v);
+    }
+    square = warp_sum(square);
+    if (lane == 0) squares[member] = square;
     __syncthreads();
-    if ((threadIdx.x & 31u) == 0) scratch[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float r = scratch[0];
-#pragma unroll
-    for (int w = 1; w < THREADS / 32; ++w) r = f(r, scratch[w]);
-    return r;
+    if (threadIdx.x) return;
+    float total = 0.0f;
+    for (uint32_t m = 0; m < members.width; ++m) total += squares[m];
+    out.scale[at] = norm_scale(total, out.columns, eps);
 }
 
-__device__ inline float4 read4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-
-// One row, in shared memory, as an operand; a thread takes four columns at a time.  The scale is the largest power of two that
-// keeps the head in f16's range, as the one-row matvecs choose it; columns are a multiple of 256, so eight lanes hold 32
-// consecutive ones.
-template <int THREADS>
-__device__ inline void split_row(const float *row, float largest, const RowsOperand &out, uint32_t at) {
-    int shift = 14 - ((int)((__float_as_uint(largest) >> 23) & 0xffu) - 127);
-    shift = max(-100, min(100, shift));
-    if (!(largest > 0.0f) || !isfinite(largest)) shift = 0;
-    const float scale = __uint_as_float((uint32_t)(shift + 127) << 23);
-    __half *head = out.split + (size_t)at * 2u * out.columns, *rest = head + out.columns;
-    for (uint32_t i = threadIdx.x * 4u; i < out.columns; i += THREADS * 4u) {
-        const float4 r = read4(row + i);
-        const float v[4] = {r.x * scale, r.y * scale, r.z * scale, r.w * scale};
-        __half2 h[2], l[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            h[j] = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
-            l[j] = __floats2half2_rn(v[2 * j] - __low2float(h[j]), v[2 * j + 1] - __high2float(h[j]));
-        }
-        *reinterpret_cast<uint2 *>(head + i) = make_uint2(*reinterpret_cast<uint32_t *>(&h[0]), *reinterpret_cast<uint32_t *>(&h[1]));
-        *reinterpret_cast<uint2 *>(rest + i) = make_uint2(*reinterpret_cast<uint32_t *>(&l[0]), *reinterpret_cast<uint32_t *>(&l[1]));
-        float s = (v[0] + v[1]) + (v[2] + v[3]);
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 7u) == 0) out.sums[(size_t)at * (out.columns / 32u) + (i >> 5)] = s;
-    }
-    if (threadIdx.x == 0) out.unscale[at] = __uint_as_float((uint32_t)(127 - shift) << 23);
+__device__ inline void store8(float *dst, const float (&v)[8]) {
+    reinterpret_cast<float4 *>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4 *>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
 }
 
-constexpr int kRowThreads = 512;
-__device__ inline float larger(float a, float b) { return fmaxf(a, b); }
-__device__ inline float added(float a, float b) { return a + b; }
-
-// rms_norm of a row in shared memory (math.rs:18-34), in place, and its operand.  Every thread its own four columns throughout.
-__device__ inline void norm_and_split(float *row, const float *w, float eps, float *normed, const RowsOperand &out, uint32_t at,
-                                      float *scratch) {
-    const uint32_t n = out.columns;
-    float s = 0.0f;
-    for (uint32_t i = threadIdx.x * 4u; i < n; i += kRowThreads * 4u) {
-        const float4 v = read4(row + i);
-        s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    }
-    const float scale = 1.0f / sqrtf(row_reduce<kRowThreads>(s, added, scratch) / (float)n + eps);
-    float mx = 0.0f;
-    for (uint32_t i = threadIdx.x * 4u; i < n; i += kRowThreads * 4u) {
-        float4 v = read4(row + i);
-        const float4 g = read4(w + i);
-        v.x = v.x * scale * g.x, v.y = v.y * scale * g.y, v.z = v.z * scale * g.z, v.w = v.w * scale * g.w;
-        *reinterpret_cast<float4 *>(row + i) = v;
-        if (normed) *reinterpret_cast<float4 *>(normed + i) = v;
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    }
-    split_row<kRowThreads>(row, row_reduce<kRowThreads>(mx, larger, scratch), out, at);
-}
-
-__global__ void __launch_bounds__(kRowThreads) moe_rows_embed_kernel(const uint32_t *tokens, const uint8_t *table, float *x,
-                                                                     const float *w, float eps, const RowsOperand out) {
-    extern __shared__ __align__(16) float row[];
-    __shared__ float scratch[kRowThreads / 32];
+__global__ void __launch_bounds__(kMaxMembers * 32) moe_rows_embed_kernel(const uint32_t *tokens, const uint8_t *table, float *x,
+                                                                          const float *w, float eps, const RowsOperand out,
+                                                                          const Members members) {
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t H = out.columns, at = blockIdx.x;
+    const uint32_t H = out.columns, at = blockIdx.x, lane = threadIdx.x & 31u;
     const uint8_t *src = table + (size_t)tokens[at] * (H / 32u) * 34u;
-    for (uint32_t i = threadIdx.x; i < H; i += kRowThreads) {
-        const uint8_t *b = src + (i >> 5) * 34u;
+    norm_operand(out, at, members, w, eps, [&](uint32_t s, float(&v)[8]) {
+        const uint32_t column = s * kSlice + lane * 8u;
+        const uint8_t *b = src + (column >> 5) * 34u;
         const float d = __half2float(__ushort_as_half((unsigned short)(b[0] | (b[1] << 8))));
-        const float v = d * (float)(int8_t)b[2u + (i & 31u)];
-        row[i] = v;
-        x[(size_t)at * H + i] = v;
-    }
-    __syncthreads();
-    norm_and_split(row, w, eps, nullptr, out, at, scratch);
-}
-
-// moe_heads_kernel for the rows of a pass: one CTA of `dim` threads per head and row.
-__global__ void moe_rows_heads_kernel(float *qkv, const float *q_norm, const float *k_norm, float *keys, float *values,
-                                      uint32_t q_heads, uint32_t kv_heads, uint32_t dim, float eps, float theta,
-                                      uint32_t first_pos) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ float scratch[32];
-    __shared__ float head[256];
-    const uint32_t h = blockIdx.x, i = threadIdx.x, position = first_pos + blockIdx.y;
-    const size_t kv_row = (size_t)kv_heads * dim;
-    float *src = qkv + ((size_t)blockIdx.y * (q_heads + 2u * kv_heads) + h) * dim;
-    if (h >= q_heads + kv_heads) {
-        values[position * kv_row + (size_t)(h - q_heads - kv_heads) * dim + i] = src[i];
-        return;
-    }
-    const float v = src[i];
-    float s = v * v;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((i & 31u) == 0) scratch[i >> 5] = s;
-    __syncthreads();
-    float sum = 0.0f;
-    for (uint32_t w = 0; w < dim / 32u; ++w) sum += scratch[w];
-    const float scale = 1.0f / sqrtf(sum / (float)dim + eps);
-    head[i] = v * scale * (h < q_heads ? q_norm : k_norm)[i];
-    __syncthreads();
-    const uint32_t half = dim / 2u, pair = i < half ? i : i - half;
-    const float angle = (float)position * powf(theta, -((float)(2u * pair)) / (float)dim);
-    float sn, cs;
-    sincosf(angle, &sn, &cs);
-    const float a = head[pair], b = head[pair + half];
-    const float out = i < half ? a * cs - b * sn : a * sn + b * cs;
-    if (h < q_heads)
-        src[i] = out;
-    else
-        keys[position * kv_row + (size_t)(h - q_heads) * dim + i] = out;
+        for (uint32_t i = 0; i < 8u; ++i) v[i] = d * (float)(int8_t)b[2u + (column & 31u) + i];
+        store8(x + (size_t)at * H + column, v);
+    });
 }
 
-// moe_attention_merge_kernel for a whole row, and the row's operand.
-__global__ void __launch_bounds__(kRowThreads) moe_rows_merge_kernel(const float *part, uint32_t splits, const RowsOperand out) {
-    constexpr uint32_t D = 128;
-    extern __shared__ __align__(16) float row[];
-    __shared__ float scratch[kRowThreads / 32];
+// Per-head norm and rope of the rows' heads and the cache rows: a warp a head, as a token's attention prepares them.
+constexpr uint32_t kHeadWarps = 4;
+__global__ void __launch_bounds__(kHeadWarps * 32) moe_rows_heads_kernel(float *qkv, const float *q_norm, const float *k_norm,
+                                                                         float *keys, float *values, uint32_t q_heads,
+                                                                         uint32_t kv_heads, float eps, float theta, uint32_t first_pos) {
+    const uint32_t lane = threadIdx.x & 31u, heads = q_heads + 2u * kv_heads, position = first_pos + blockIdx.y;
+    const uint32_t h = blockIdx.x * kHeadWarps + (threadIdx.x >> 5);
     pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t heads = out.columns / D;
-    float mx = 0.0f;
-    for (uint32_t i = threadIdx.x; i < out.columns; i += kRowThreads) {
-        const float *src = part + ((size_t)blockIdx.x * heads + i / D) * splits * (D + 2u);
-        float gm = -INFINITY;
-        for (uint32_t s = 0; s < splits; ++s) gm = fmaxf(gm, src[s * (D + 2u)]);
-        float l = 0.0f, a = 0.0f;
-        for (uint32_t s = 0; s < splits; ++s) {
-            const float m = src[s * (D + 2u)];
-            const float c = m == -INFINITY ? 0.0f : expf(m - gm);  // an empty span weighs nothing
-            l += src[s * (D + 2u) + 1u] * c;
-            a += src[s * (D + 2u) + 2u + i % D] * c;
-        }
-        const float v = a / l;
-        row[i] = v;
-        mx = fmaxf(mx, fabsf(v));
+    float norm[4], cs[2], sn[2], v[4], o[4];
+    if (h < q_heads + kv_heads) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) norm[k] = (h < q_heads ? q_norm : k_norm)[32 * k + lane];
+        head_angles(position, theta, lane, cs, sn);
     }
-    split_row<kRowThreads>(row, row_reduce<kRowThreads>(mx, larger, scratch), out, blockIdx.x);
+    pdl_wait();
+    if (h >= heads) return;
+    float *src = qkv + ((size_t)blockIdx.y * heads + h) * kHeadWidth, *dst = src;
+    const size_t cache_row = (size_t)position * kv_heads * kHeadWidth;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k] = v[k] = src[32 * k + lane];
+    if (h < q_heads + kv_heads) prepare_head(v, norm, cs, sn, eps, o);
+    if (h >= q_heads + kv_heads) dst = values + cache_row + (size_t)(h - q_heads - kv_heads) * kHeadWidth;
+    else if (h >= q_heads) dst = keys + cache_row + (size_t)(h - q_heads) * kHeadWidth;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) dst[32 * k + lane] = o[k];
 }
 
-__global__ void __launch_bounds__(kRowThreads) moe_rows_add_norm_kernel(float *x, const float *update, const float *probs,
-                                                                        uint32_t active, const float *w, float eps, float *normed,
-                                                                        const RowsOperand out, uint32_t hidden) {
-    extern __shared__ __align__(16) float row[];
-    __shared__ float scratch[kRowThreads / 32];
-    __shared__ float share[32];
+// G values a lane, each summed over the warp as warp_sum does it: the same pairs in the same order, but a lane goes on with half
+// of the values at a time.  Returns value lane / (32 / G).
+template <int G>
+__device__ inline float group_sums(float (&d)[G], uint32_t lane) {
+    int left = G;
+#pragma unroll
+    for (uint32_t o = 16u; o > 0; o >>= 1) {
+        if (left > 1) {
+            left /= 2;
+#pragma unroll
+            for (int i = 0; i < G / 2; ++i)
+                if (i < left) {
+                    const float got = __shfl_xor_sync(0xffffffffu, lane & o ? d[i] : d[i + left], o);
+                    d[i] = (lane & o ? d[i + left] : d[i]) + got;
+                }
+        } else {
+            d[0] += __shfl_xor_sync(0xffffffffu, d[0], o);
+        }
+    }
+    return d[0];
+}
+
+// State of a span of a head: its maximum and sum, two unused words, its 128 columns.
+constexpr uint32_t kSpanState = kHeadWidth + 4u;
+
+// Attention of a row, `each` spans of a KV head a CTA: as in a token a warp is a strand, which reads a key once for the G query
+// heads of the group; 32 / G lanes keep the maximum and sum of a head.  Bound by instruction issue.
+template <int G>
+__global__ void __launch_bounds__(kStrands * 32, 2) moe_rows_attention_kernel(const float *qkv, const float *keys, const float *values,
+                                                                              float *part, uint32_t first_pos, uint32_t splits,
+                                                                              uint32_t each, uint32_t spans, uint32_t kv_heads, float scale) {
+    constexpr uint32_t kLanes = 32u / G;
+    __shared__ float sm[kStrands][G], sl[kStrands][G];
+    __shared__ __align__(16) float4 sacc[kStrands][G][32];
+    const uint32_t kvh = blockIdx.x, row = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t rows = first_pos + row + 1u, span = span_rows(rows, splits), used = (rows + span - 1u) / span;
+    const uint32_t from = blockIdx.y * each, to = min(used, from + each);
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t at = blockIdx.x;
-    if (probs && threadIdx.x < active) share[threadIdx.x] = probs[(size_t)at * active + threadIdx.x];
-    __syncthreads();
+    if (from >= to) return;
+    const size_t kv_row = (size_t)kv_heads * kHeadWidth;
+    const auto fetch = [&](const float *cache, uint32_t t) {
+        return reinterpret_cast<const float4 *>(cache + min(t, rows - 1u) * kv_row + kvh * kHeadWidth)[lane];
+    };
+    float4 q[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+        q[g] = reinterpret_cast<const float4 *>(qkv + ((size_t)row * kv_heads * (G + 2u) + kvh * G + g) * kHeadWidth)[lane];
+    float4 k = fetch(keys, from * span + warp), v = fetch(values, from * span + warp);
+    for (uint32_t n = from; n < to; ++n) {
+        const uint32_t lo = n * span, hi = min(rows, lo + span);
+        float m = -INFINITY, l = 0.0f;
+        float4 acc[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) acc[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (uint32_t t = lo + warp; t < hi; t += kStrands) {
+            const float4 now = k, value = v;
+            const uint32_t next = t + kStrands < hi ? t + kStrands : hi + warp;  // of this span, or the first of the next
+            k = fetch(keys, next), v = fetch(values, next);
+            float dot[G], c, e;
+#pragma unroll
+            for (int g = 0; g < G; ++g) dot[g] = dot4(q[g], now);
+            strand_step(m, l, __fmul_rn(group_sums<G>(dot, lane), scale), c, e);
+#pragma unroll
+            for (int g = 0; g < G; ++g) strand_add(acc[g], __shfl_sync(0xffffffffu, c, g * kLanes), __shfl_sync(0xffffffffu, e, g * kLanes), value);
+        }
+        __syncthreads();  // the span before this one has been merged
+        if (lane % kLanes == 0) sm[warp][lane / kLanes] = m, sl[warp][lane / kLanes] = l;
+#pragma unroll
+        for (int g = 0; g < G; ++g) sacc[warp][g][lane] = acc[g];
+        __syncthreads();
+        if (warp >= (uint32_t)G) continue;
+        float top = -INFINITY, sum = 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < kStrands; ++w) top = fmaxf(top, sm[w][warp]);
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (uint32_t w = 0; w < kStrands; ++w) strand_take(sum, a, strand_weight(sm[w][warp], top), sl[w][warp], sacc[w][warp][lane]);
+        float *dst = part + (((size_t)row * kv_heads * G + kvh * G + warp) * spans + n) * kSpanState;
+        if (lane == 0) *reinterpret_cast<float2 *>(dst) = make_float2(top, sum);
+        reinterpret_cast<float4 *>(dst)[lane + 1u] = a;
+    }
+}
+
+// Merges the spans of a row's heads: a slice is two heads, half a warp each.
+constexpr uint32_t kMergeWarps = 4;
+__global__ void __launch_bounds__(kMergeWarps * 32) moe_rows_merge_kernel(const float *part, uint32_t first_pos, uint32_t splits,
+                                                                          uint32_t spans, uint32_t first_row, const RowsOperand out) {
+    const uint32_t lane = threadIdx.x & 31u, row = blockIdx.x, heads = out.columns / kHeadWidth;
+    const uint32_t s = blockIdx.y * kMergeWarps + (threadIdx.x >> 5);
+    const uint32_t rows = first_pos + row + 1u, span = span_rows(rows, splits), used = (rows + span - 1u) / span;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (2u * s >= heads) return;
+    const float *src = part + ((size_t)row * heads + 2u * s) * spans * kSpanState;
+    float c[2][2], total[2];
+#pragma unroll
+    for (uint32_t h = 0; h < 2u; ++h) {
+        float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (uint32_t j = 0; j < 2u; ++j)
+            if (lane + 32u * j < used) {
+                const float2 state = *reinterpret_cast<const float2 *>(src + ((size_t)h * spans + lane + 32u * j) * kSpanState);
+                m[j] = state.x, l[j] = state.y;
+            }
+        total[h] = span_weights(m, l, c[h]);
+    }
+    const bool second = lane >= 16u;
+    src += (second ? spans * kSpanState : 0u) + 4u + (lane & 15u) * 8u;
+    float v[8] = {};
+#pragma unroll 8
+    for (uint32_t n = 0; n < used; ++n) {
+        const float first_weight = __shfl_sync(0xffffffffu, n < 32u ? c[0][0] : c[0][1], n & 31u);
+        const float second_weight = __shfl_sync(0xffffffffu, n < 32u ? c[1][0] : c[1][1], n & 31u);
+        const float weight = second ? second_weight : first_weight;
+        float a[8];
+        load8(src + n * kSpanState, a);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = fmaf(a[i], weight, v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = v[i] / (second ? total[1] : total[0]);
+    store_slice(out, first_row + row, s, v);
+}
+
+__global__ void __launch_bounds__(kMaxMembers * 32) moe_rows_add_norm_kernel(float *x, const float *update, const float *probs,
+                                                                             uint32_t active, const float *w, float eps,
+                                                                             const RowsOperand out, const Members members) {
+    __shared__ float share[32];
+    const uint32_t at = blockIdx.x, lane = threadIdx.x & 31u, hidden = out.columns;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (probs) {
+        for (uint32_t e = threadIdx.x; e < active; e += blockDim.x) share[e] = probs[(size_t)at * active + e];
+        __syncthreads();
+    }
     const float *rows = update + (size_t)at * (probs ? active : 1u) * hidden;
-    for (uint32_t i = threadIdx.x * 4u; i < hidden; i += kRowThreads * 4u) {
-        float4 *home = reinterpret_cast<float4 *>(x + (size_t)at * hidden + i);
-        float4 v = *home, r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    norm_operand(out, at, members, w, eps, [&](uint32_t s, float(&v)[8]) {
+        const uint32_t column = s * kSlice + lane * 8u;
+        float *home = x + (size_t)at * hidden + column, r[8], o[8];
+        load8(home, v);
         if (probs) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] = 0.0f;
 #pragma unroll 8
             for (uint32_t e = 0; e < active; ++e) {
-                const float4 o = read4(rows + (size_t)e * hidden + i);
-                r.x += share[e] * o.x, r.y += share[e] * o.y, r.z += share[e] * o.z, r.w += share[e] * o.w;
+                load8(rows + (size_t)e * hidden + column, o);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) r[i] = fmaf(share[e], o[i], r[i]);
             }
         } else {
-            r = read4(rows + i);
+            load8(rows + column, r);
         }
-        v.x += r.x, v.y += r.y, v.z += r.z, v.w += r.w;
-        *home = v;
-        *reinterpret_cast<float4 *>(row + i) = v;
-    }
-    if (w) norm_and_split(row, w, eps, normed ? normed + (size_t)at * hidden : nullptr, out, at, scratch);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] += r[i];
+        store8(home, v);
+    });
 }
 
-// Router scores of four rows and kRouteWarps experts a CTA: a warp multiplies one router row with the four.  (All experts of
-// four rows in one CTA took 40 us: the 1 MB of router rows went by one after another.)
-constexpr uint32_t kRouteRows = 4, kRouteWarps = 8;
-__global__ void __launch_bounds__(kRouteWarps * 32) moe_rows_scores_kernel(const float *router, const float *normed, uint32_t hidden,
-                                                                           uint32_t experts, float *scores, uint32_t rows) {
-    pdl_launch_dependents();
-    const uint32_t lane = threadIdx.x & 31u, e = blockIdx.y * kRouteWarps + (threadIdx.x >> 5), first = blockIdx.x * kRouteRows;
-    if (e >= experts) {
-        pdl_wait();
-        return;
-    }
-    const float4 *w = reinterpret_cast<const float4 *>(router + (size_t)e * hidden);
-    const float4 *x[kRouteRows];
+// Router scores of 16 rows and four experts a CTA, a warp a member of the rows: it holds its slice of the four experts' rows
+// times the norm's weights, so an input row is read once for four scores.  (All experts of four rows in one CTA took 40 us: the
+// 1 MB of router rows went by one after another.)
+constexpr uint32_t kRouteRows = 16, kRouteExperts = 4;
+__global__ void __launch_bounds__(kMaxMembers * 32) moe_rows_scores_kernel(const float *router, const float *x, const float *norm,
+                                                                           const float *scale, uint32_t experts, float *scores,
+                                                                           uint32_t rows, const Members at) {
+    __shared__ float part[kRouteRows][kRouteExperts][kMaxMembers];
+    const uint32_t lane = threadIdx.x & 31u, member = threadIdx.x >> 5, expert0 = blockIdx.x * kRouteExperts, row0 = blockIdx.y * kRouteRows;
+    const uint32_t hidden = at.supers * kSlice, count = min(kRouteRows, rows - row0);
+    float a[kRouteExperts][8];
+    const auto products = [&](uint32_t s) {
+        float w[8];
+        load8(norm + s * kSlice + lane * 8u, w);
 #pragma unroll
-    for (uint32_t r = 0; r < kRouteRows; ++r)
-        x[r] = reinterpret_cast<const float4 *>(normed + (size_t)min(first + r, rows - 1u) * hidden);
-    constexpr uint32_t kAhead = 4;
-    float4 a[kAhead];
-    const auto fetch = [&](uint32_t from) {
+        for (uint32_t e = 0; e < kRouteExperts; ++e) {
+            load8(router + (size_t)min(expert0 + e, experts - 1u) * hidden + s * kSlice + lane * 8u, a[e]);
 #pragma unroll
-        for (uint32_t j = 0; j < kAhead; ++j)
-            if (from + 32u * j < hidden / 4u) a[j] = w[from + 32u * j];
-    };
-    fetch(lane);
-    pdl_wait();
-    float s[kRouteRows] = {};
-    for (uint32_t from = lane; from < hidden / 4u; from += 32u * kAhead) {
-        float4 now[kAhead];
-#pragma unroll
-        for (uint32_t j = 0; j < kAhead; ++j) now[j] = a[j];
-        fetch(from + 32u * kAhead);
-#pragma unroll
-        for (uint32_t j = 0; j < kAhead; ++j) {
-            const uint32_t i = from + 32u * j;
-            if (i >= hidden / 4u) break;
-#pragma unroll
-            for (uint32_t r = 0; r < kRouteRows; ++r) {
-                const float4 b = x[r][i];
-                s[r] += now[j].x * b.x + now[j].y * b.y + now[j].z * b.z + now[j].w * b.w;
-            }
+            for (int i = 0; i < 8; ++i) a[e][i] = __fmul_rn(a[e][i], w[i]);
         }
-    }
+    };
+    pdl_launch_dependents();
+    products(member);
+    pdl_wait();
+#pragma unroll 2
+    for (uint32_t row = 0; row < count; ++row) {
+        float dot[kRouteExperts] = {};
+        for (uint32_t s = member; s < at.supers; s += at.width) {
+            float v[8];
+            if (at.records > 1u) products(s);
+            load8(x + (size_t)(row0 + row) * hidden + s * kSlice + lane * 8u, v);
 #pragma unroll
-    for (uint32_t r = 0; r < kRouteRows; ++r) {
-        s[r] = warp_sum(s[r]);
-        if (lane == 0 && first + r < rows) scores[(size_t)(first + r) * experts + e] = s[r];
+            for (uint32_t e = 0; e < kRouteExperts; ++e)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dot[e] = fmaf(a[e][i], v[i], dot[e]);
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < kRouteExperts; ++e) dot[e] = warp_sum(dot[e]);
+        if (lane == 0)
+#pragma unroll
+            for (uint32_t e = 0; e < kRouteExperts; ++e) part[row][e][member] = dot[e];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < count * kRouteExperts; i += blockDim.x) {
+        const uint32_t row = i / kRouteExperts, e = i % kRouteExperts;
+        if (expert0 + e >= experts) continue;
+        float dot = 0.0f;
+        for (uint32_t m = 0; m < at.width; ++m) dot += part[row][e][m];
+        scores[(size_t)(row0 + row) * experts + expert0 + e] = __fmul_rn(dot, scale[row0 + row]);
     }
 }
 
@@ -477,74 +586,47 @@ __global__ void __launch_bounds__(kListThreads) moe_rows_lists_kernel(const uint
     for (uint32_t i = tid; i < count; i += kListThreads) pairs[starts[ids[i]] + atomicAdd(&counts[ids[i]], 1u)] = i;
 }
 
-constexpr int kGateThreads = 256;
-__global__ void __launch_bounds__(kGateThreads) moe_rows_gate_kernel(const float *gate_up, const RowsOperand out) {
-    extern __shared__ __align__(16) float row[];
-    __shared__ float scratch[kGateThreads / 32];
+// silu(gate) * up of every pair, a warp a slice.
+constexpr uint32_t kGateWarps = 8;
+__global__ void __launch_bounds__(kGateWarps * 32) moe_rows_gate_kernel(const float *gate_up, const RowsOperand out, uint32_t slices) {
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t I = out.columns;
-    const float *gate = gate_up + (size_t)blockIdx.x * 2u * I, *up = gate + I;
-    float mx = 0.0f;
-    for (uint32_t i = threadIdx.x; i < I; i += kGateThreads) {  // silu with the two-branch sigmoid (math.rs:5-16)
-        const float g = gate[i];
-        float sg;
-        if (g >= 0.0f) {
-            sg = 1.0f / (1.0f + expf(-g));
-        } else {
-            const float e = expf(g);
-            sg = e / (1.0f + e);
-        }
-        const float v = g * sg * up[i];
-        row[i] = v;
-        mx = fmaxf(mx, fabsf(v));
-    }
-    split_row<kGateThreads>(row, row_reduce<kGateThreads>(mx, larger, scratch), out, blockIdx.x);
+    const uint32_t lane = threadIdx.x & 31u, i = blockIdx.x * kGateWarps + (threadIdx.x >> 5), each = out.columns / kSlice;
+    if (i >= slices) return;
+    const float *gates = gate_up + (size_t)(i / each) * 2u * out.columns + i % each * kSlice + lane * 8u;
+    float g[8], u[8], v[8];
+    load8(gates, g), load8(gates + out.columns, u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = gated_value(g[j], u[j]);
+    store_slice(out, i / each, i % each, v);
 }
 
-// A launch that may start before its predecessor ends: every kernel here awaits it before its first access.
+// Launches that may start before their predecessor ends: every kernel here awaits it before its first access to what it made.
 template <typename... Params, typename... Args>
 stark_b200_status launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    SB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
-    return STARK_B200_OK;
+    return moe_launch(kernel, grid, block, smem, true, stream, args...);
 }
 
-// The kernels that hold a row in shared memory: the widest takes 48 KB beside their own words, more than a launch has unasked.
-template <typename... Params, typename... Args>
-stark_b200_status launch_row(SmemOptIn &once, void (*kernel)(Params...), dim3 grid, dim3 block, uint32_t columns, cudaStream_t stream,
-                             Args... args) {
-    if (columns > kMoeRowsWidest) return STARK_B200_UNSUPPORTED;
-    if (stark_b200_status s = ensure_dynamic_smem(kernel, (int)kMoeRowsWidest * 4, once)) return s;
-    return launch(kernel, grid, block, (size_t)columns * 4u, stream, args...);
-}
+// CTAs of a pass's attention from which on each takes more than one span.
+constexpr uint32_t kAttentionCtas = 1184;
 
-constexpr size_t gemm_smem(uint32_t stages, uint32_t warps, uint32_t super_bytes, uint32_t sums) {
-    return stages * (warps * super_bytes + kTileLines * kLine + sums);
+constexpr size_t gemm_smem(uint32_t stages, uint32_t warps, bool q4) {
+    return stages * (warps * (q4 ? kQ4SuperBytes : kB8SuperBytes) + kTileLines * kLine + kMoeRowsChunk * (q4 ? kMetaBytes<true> : kMetaBytes<false>));
 }
 constexpr uint32_t kQ4Stages = 3, kQ4Warps = 8;
-constexpr size_t kQ4Smem = gemm_smem(kQ4Stages, kQ4Warps, kQ4SuperBytes, kMoeRowsChunk * 32u);
+constexpr size_t kQ4Smem = gemm_smem(kQ4Stages, kQ4Warps, true);
 
 RowsGemmParams gemm_params(const QMatrix *w, uint32_t super_bytes, uint32_t warps, const RowsOperand &x, float *out) {
     RowsGemmParams p{};
     p.data = w->data;
     p.rows = w->rows;
     p.row_tiles = w->row_tiles;
-    p.supers = w->columns / 256u;
+    p.at = members_of(w->columns);
     p.row_blocks = (w->row_tiles + warps - 1u) / warps;
-    p.matrix_bytes = (size_t)w->row_tiles * p.supers * super_bytes;
+    p.matrix_bytes = (size_t)w->row_tiles * p.at.supers * super_bytes;
     p.x = x.split;
-    p.unscale = x.unscale;
-    p.sums = x.sums;
+    p.meta = x.meta;
+    p.scale = x.scale;
     p.out = out;
     p.divisor = 1;
     return p;
@@ -559,11 +641,13 @@ stark_b200_status rows_q8_launch(const QMatrix *w, const RowsOperand &x, float *
     const uint32_t chunks = (rows + kMoeRowsChunk - 1u) / kMoeRowsChunk;
     const bool narrow = (w->row_tiles + 7u) / 8u * chunks < 148u;
     const uint32_t warps = narrow ? 2u : 8u;
-    const size_t smem = gemm_smem(narrow ? 4u : 2u, warps, kB8SuperBytes, 0u);
-    const auto kernel = narrow ? rows_gemm_kernel<false, 4, 2> : rows_gemm_kernel<false, 2, 8>;
-    static SmemOptIn once[2];
-    if (stark_b200_status s = ensure_dynamic_smem(kernel, (int)smem, once[narrow])) return s;
+    const size_t smem = gemm_smem(narrow ? 4u : 2u, warps, false);
     RowsGemmParams p = gemm_params(w, kB8SuperBytes, warps, x, out);
+    const bool multi = p.at.records > 1u;
+    const auto kernel = narrow ? (multi ? rows_gemm_kernel<false, 4, 2, true> : rows_gemm_kernel<false, 4, 2, false>)
+                               : (multi ? rows_gemm_kernel<false, 2, 8, true> : rows_gemm_kernel<false, 2, 8, false>);
+    static SmemOptIn once[2][2];
+    if (stark_b200_status s = ensure_dynamic_smem(kernel, (int)smem, once[narrow][multi])) return s;
     p.m = rows;
     p.out_stride = w->rows;
     return launch(kernel, dim3(p.row_blocks, chunks), warps * 32u, smem, stream, p);
@@ -572,51 +656,67 @@ stark_b200_status rows_q8_launch(const QMatrix *w, const RowsOperand &x, float *
 stark_b200_status rows_q4k_experts_launch(const QMatrix *w, uint32_t blocks, const RowsOperand &x, uint32_t divisor, float *out,
                                           const MoeRowLists &lists, uint32_t rows, uint32_t active, cudaStream_t stream) {
     if (w->format != kFmtQ4_K || w->columns != x.columns || rows == 0 || w->experts % blocks) return STARK_B200_INVALID_ARGUMENT;
-    static SmemOptIn once;
-    if (stark_b200_status s = ensure_dynamic_smem(rows_gemm_kernel<true, kQ4Stages, kQ4Warps>, (int)kQ4Smem, once)) return s;
     RowsGemmParams p = gemm_params(w, kQ4SuperBytes, kQ4Warps, x, out);
+    const bool multi = p.at.records > 1u;
+    const auto kernel = multi ? rows_gemm_kernel<true, kQ4Stages, kQ4Warps, true> : rows_gemm_kernel<true, kQ4Stages, kQ4Warps, false>;
+    static SmemOptIn once[2];
+    if (stark_b200_status s = ensure_dynamic_smem(kernel, (int)kQ4Smem, once[multi])) return s;
     p.experts = w->experts / blocks;
     p.tiles = lists.tiles;
     p.pairs = lists.pairs;
     p.divisor = divisor;
     p.out_stride = blocks * w->rows;
-    return launch(rows_gemm_kernel<true, kQ4Stages, kQ4Warps>, dim3(p.row_blocks * blocks, MoeRowLists::max_tiles(rows, active, p.experts)),
+    return launch(kernel, dim3(p.row_blocks * blocks, MoeRowLists::max_tiles(rows, active, p.experts)),
                   kQ4Warps * 32u, kQ4Smem, stream, p);
 }
 
 stark_b200_status moe_rows_embed_launch(const uint32_t *tokens, const uint8_t *table, float *x, const float *w, float eps,
                                         const RowsOperand &out, uint32_t rows, cudaStream_t stream) {
-    static SmemOptIn once;
-    return launch_row(once, moe_rows_embed_kernel, rows, kRowThreads, out.columns, stream, tokens, table, x, w, eps, out);
+    const Members at = members_of(out.columns);
+    return launch(moe_rows_embed_kernel, rows, at.width * 32u, 0, stream, tokens, table, x, w, eps, out, at);
 }
 
 stark_b200_status moe_rows_heads_launch(float *qkv, const float *q_norm, const float *k_norm, float *keys, float *values,
-                                        uint32_t q_heads, uint32_t kv_heads, uint32_t dim, float eps, float theta,
-                                        uint32_t first_pos, uint32_t rows, cudaStream_t stream) {
-    return launch(moe_rows_heads_kernel, dim3(q_heads + 2u * kv_heads, rows), dim, 0, stream, qkv, q_norm, k_norm, keys, values,
-                  q_heads, kv_heads, dim, eps, theta, first_pos);
+                                        uint32_t q_heads, uint32_t kv_heads, float eps, float theta, uint32_t first_pos,
+                                        uint32_t rows, cudaStream_t stream) {
+    return launch(moe_rows_heads_kernel, dim3((q_heads + 2u * kv_heads + kHeadWarps - 1u) / kHeadWarps, rows), kHeadWarps * 32u, 0, stream,
+                  qkv, q_norm, k_norm, keys, values, q_heads, kv_heads, eps, theta, first_pos);
 }
 
-stark_b200_status moe_rows_merge_launch(const float *part, uint32_t heads, uint32_t splits, const RowsOperand &out,
-                                        uint32_t rows, cudaStream_t stream) {
-    if (out.columns != heads * 128u) return STARK_B200_INVALID_ARGUMENT;
-    static SmemOptIn once;
-    return launch_row(once, moe_rows_merge_kernel, rows, kRowThreads, out.columns, stream, part, splits, out);
+stark_b200_status moe_rows_attention_launch(const float *qkv, const float *keys, const float *values, float *part, size_t part_floats,
+                                            uint32_t q_heads, uint32_t kv_heads, uint32_t splits, uint32_t first_pos,
+                                            const RowsOperand &out, uint32_t rows, cudaStream_t stream) {
+    const uint32_t group = q_heads / kv_heads, spans = moe_rows_spans(splits, first_pos + rows);
+    const size_t row_floats = moe_rows_part(q_heads, spans);
+    if (out.columns != q_heads * kHeadWidth || splits > 64u || part_floats < row_floats) return STARK_B200_INVALID_ARGUMENT;
+    const auto kernel = group == 8u ? moe_rows_attention_kernel<8> : (group == 4u ? moe_rows_attention_kernel<4> : moe_rows_attention_kernel<2>);
+    const uint32_t batch = (uint32_t)std::min<size_t>(rows, part_floats / row_floats);
+    for (uint32_t done = 0; done < rows; done += batch) {
+        const uint32_t now = std::min(batch, rows - done), pos = first_pos + done;
+        const uint32_t each = std::max(1u, std::min(spans, kv_heads * spans * now / kAttentionCtas));
+        if (stark_b200_status s = launch(kernel, dim3(kv_heads, (spans + each - 1u) / each, now), kStrands * 32u, 0, stream,
+                                         qkv + (size_t)done * (q_heads + 2u * kv_heads) * kHeadWidth, keys, values, part, pos, splits, each,
+                                         spans, kv_heads, 1.0f / sqrtf((float)kHeadWidth)))
+            return s;
+        if (stark_b200_status s = launch(moe_rows_merge_kernel, dim3(now, (q_heads / 2u + kMergeWarps - 1u) / kMergeWarps), kMergeWarps * 32u, 0, stream,
+                                         part, pos, splits, spans, done, out))
+            return s;
+    }
+    return STARK_B200_OK;
 }
 
 stark_b200_status moe_rows_add_norm_launch(float *x, const float *update, const float *probs, uint32_t active, const float *w,
-                                           float eps, float *normed, const RowsOperand &out, uint32_t rows, uint32_t hidden,
-                                           cudaStream_t stream) {
-    static SmemOptIn once;
-    return launch_row(once, moe_rows_add_norm_kernel, rows, kRowThreads, hidden, stream, x, update, probs, active, w, eps,
-                  normed, out, hidden);
+                                           float eps, const RowsOperand &out, uint32_t rows, cudaStream_t stream) {
+    const Members at = members_of(out.columns);
+    return launch(moe_rows_add_norm_kernel, rows, at.width * 32u, 0, stream, x, update, probs, active, w, eps, out, at);
 }
 
-stark_b200_status moe_rows_route_launch(const float *router, const float *normed, uint32_t hidden, uint32_t experts,
-                                        uint32_t active, const MoeRowLists &lists, uint32_t *last_ids, uint32_t rows,
-                                        cudaStream_t stream) {
-    if (stark_b200_status s = launch(moe_rows_scores_kernel, dim3((rows + kRouteRows - 1u) / kRouteRows, (experts + kRouteWarps - 1u) / kRouteWarps),
-                                     kRouteWarps * 32u, 0, stream, router, normed, hidden, experts, lists.scores, rows))
+stark_b200_status moe_rows_route_launch(const float *router, const float *x, const float *norm, const RowsOperand &normed,
+                                        uint32_t experts, uint32_t active, const MoeRowLists &lists, uint32_t *last_ids,
+                                        uint32_t rows, cudaStream_t stream) {
+    const Members at = members_of(normed.columns);
+    if (stark_b200_status s = launch(moe_rows_scores_kernel, dim3((experts + kRouteExperts - 1u) / kRouteExperts, (rows + kRouteRows - 1u) / kRouteRows),
+                                     at.width * 32u, 0, stream, router, x, norm, normed.scale, experts, lists.scores, rows, at))
         return s;
     return launch(experts <= 128u ? moe_rows_select_kernel<4> : moe_rows_select_kernel<32>, (rows + kSelectWarps - 1u) / kSelectWarps,
                   kSelectWarps * 32u, 0, stream, lists.scores, experts, active, lists.ids, lists.probs, last_ids, rows);
@@ -627,10 +727,11 @@ stark_b200_status moe_rows_lists_launch(const MoeRowLists &lists, uint32_t rows,
     return launch(moe_rows_lists_kernel, 1, kListThreads, 0, stream, lists.ids, lists.pairs, lists.tiles, rows * active, experts);
 }
 
-stark_b200_status moe_rows_gate_launch(const float *gate_up, uint32_t inter, const RowsOperand &out, uint32_t pairs,
-                                       cudaStream_t stream) {
-    static SmemOptIn once;
-    return launch_row(once, moe_rows_gate_kernel, pairs, kGateThreads, inter, stream, gate_up, out);
+stark_b200_status moe_rows_gate_launch(const float *gate_up, const RowsOperand &out, uint32_t pairs, cudaStream_t stream) {
+    const uint32_t slices = pairs * (out.columns / kSlice);
+    return launch(moe_rows_gate_kernel, (slices + kGateWarps - 1u) / kGateWarps, kGateWarps * 32u, 0, stream, gate_up, out, slices);
 }
+
+size_t moe_rows_part(uint32_t q_heads, uint32_t spans) { return (size_t)q_heads * spans * kSpanState; }
 
 }  // namespace sb

@@ -17,7 +17,7 @@
 #include <cmath>
 
 #include "context.cuh"
-#include "gguf_math.cuh"
+#include "moe_math.cuh"
 #include "moe_select.cuh"
 #include "moe_token.cuh"
 
@@ -25,45 +25,32 @@ namespace sb {
 
 namespace {
 
-constexpr uint32_t kDim = 128;              // head dimension
+constexpr uint32_t kDim = kHeadWidth;
 constexpr uint32_t kSliceLine = 512 + 64;   // head or remainder of 256 inputs: two lines 64 B apart modulo 128 B
 constexpr uint32_t kSliceBytes = 2 * kSliceLine;
-constexpr uint32_t kMaxWarps = 16;
+constexpr uint32_t kMaxWarps = kMaxMembers;
 
-// The eight inputs of a lane (8 lane ... + 7 of a slice of 256) as f16 head and remainder of v * 2^s, s by the slice's largest
-// element; returns 2^-s.  xa, xb: sums of v over the sub-blocks t and t + 4 (32 columns each).
+// The eight inputs of a lane (8 lane ... + 7 of a slice) as the products read them; returns 2^-s.  xa, xb: sums of the scaled
+// slice over the sub-blocks t and t + 4 (32 columns each).
 __device__ inline float stage_slice(const float (&v)[8], uint8_t *lines, uint32_t lane, float &xa, float &xb) {
-    uint32_t top = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) top = max(top, __float_as_uint(v[i]) & 0x7fffffffu);
-    top = __reduce_max_sync(0xffffffffu, top);
-    int shift = max(-100, min(100, 14 - ((int)(top >> 23) - 127)));
-    if (top == 0u || top >= 0x7f800000u) shift = 0;
-    const float scale = __uint_as_float((uint32_t)(shift + 127) << 23);
-    uint32_t head[4], rest[4];
-    float sum = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float a = v[2 * i] * scale, b = v[2 * i + 1] * scale;
-        const __half2 h = __floats2half2_rn(a, b), r = __floats2half2_rn(a - __low2float(h), b - __high2float(h));
-        head[i] = *reinterpret_cast<const uint32_t *>(&h);
-        rest[i] = *reinterpret_cast<const uint32_t *>(&r);
-        sum += v[2 * i] + v[2 * i + 1];
-    }
+    const SplitSlice s = split_slice(v);
     __syncwarp();  // the slice before this one has been read
-    *reinterpret_cast<uint4 *>(lines + lane * 16u) = make_uint4(head[0], head[1], head[2], head[3]);
-    *reinterpret_cast<uint4 *>(lines + kSliceLine + lane * 16u) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    *reinterpret_cast<uint4 *>(lines + lane * 16u) = s.head;
+    *reinterpret_cast<uint4 *>(lines + kSliceLine + lane * 16u) = s.rest;
     const uint32_t t = lane & 3u;
-    xa = __shfl_sync(0xffffffffu, sum, 4u * t);
-    xb = __shfl_sync(0xffffffffu, sum, 4u * t + 16u);
+    xa = __shfl_sync(0xffffffffu, s.sum, 4u * t);
+    xb = __shfl_sync(0xffffffffu, s.sum, 4u * t + 16u);
     __syncwarp();
-    return __uint_as_float((uint32_t)(127 - shift) << 23);
+    return s.down;
 }
 
-// A record times the staged slice: this lane's share (sub-blocks t and t + 4) of rows g and g + 8, added to v0 and v1.
-__device__ inline void q8_record(const uint8_t *rec, const uint8_t *lines, float unscale, uint32_t lane, float &v0, float &v1) {
+__device__ inline float quad_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// A record times the staged slice, added to the sums of rows g and g + 8 (on all four lanes of a row).
+__device__ inline void q8_record(const uint8_t *rec, const uint8_t *lines, float down, uint32_t lane, float &v0, float &v1) {
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint16_t *meta = reinterpret_cast<const uint16_t *>(rec + 4096u);
     const uint8_t *x = lines + (g & 1u) * kSliceLine + t * 16u;  // column n = g of B: even the head, odd the remainder
@@ -84,11 +71,12 @@ __device__ inline void q8_record(const uint8_t *rec, const uint8_t *lines, float
         s0[jb >> 2] = mine ? c[0] + c[1] : s0[jb >> 2];
         s1[jb >> 2] = mine ? c[2] + c[3] : s1[jb >> 2];
     }
-    v0 = fmaf(unscale, fmaf(f16_bits_f32(meta[t * 16u + g]), s0[0], f16_bits_f32(meta[(t + 4u) * 16u + g]) * s0[1]), v0);
-    v1 = fmaf(unscale, fmaf(f16_bits_f32(meta[t * 16u + g + 8u]), s1[0], f16_bits_f32(meta[(t + 4u) * 16u + g + 8u]) * s1[1]), v1);
+    const float r0 = q8_share(f16_bits_f32(meta[t * 16u + g]), s0[0], f16_bits_f32(meta[(t + 4u) * 16u + g]), s0[1]);
+    const float r1 = q8_share(f16_bits_f32(meta[t * 16u + g + 8u]), s1[0], f16_bits_f32(meta[(t + 4u) * 16u + g + 8u]), s1[1]);
+    v0 = fmaf(down, quad_sum(r0), v0), v1 = fmaf(down, quad_sum(r1), v1);
 }
 
-__device__ inline void q4_record(const uint8_t *rec, const uint8_t *lines, float unscale, float xa, float xb, uint32_t lane,
+__device__ inline void q4_record(const uint8_t *rec, const uint8_t *lines, float down, float xa, float xb, uint32_t lane,
                                  float &v0, float &v1) {
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint8_t *x = lines + (g & 1u) * kSliceLine + t * 16u;
@@ -109,9 +97,10 @@ __device__ inline void q4_record(const uint8_t *rec, const uint8_t *lines, float
     }
     float dsc[2], dm[2];
     q4k_scales_pair(*reinterpret_cast<const uint4 *>(rec + 2048u + 16u * g), t, dsc, dm);
-    v0 = fmaf(unscale, fmaf(dsc[0], s0[0], dsc[1] * s0[1]), v0) - fmaf(dm[0], xa, dm[1] * xb);
+    const float r0 = q4k_share(dsc[0], s0[0], dsc[1], s0[1], dm[0], xa, dm[1], xb);
     q4k_scales_pair(*reinterpret_cast<const uint4 *>(rec + 2048u + 16u * (g + 8u)), t, dsc, dm);
-    v1 = fmaf(unscale, fmaf(dsc[0], s1[0], dsc[1] * s1[1]), v1) - fmaf(dm[0], xa, dm[1] * xb);
+    const float r1 = q4k_share(dsc[0], s1[0], dsc[1], s1[1], dm[0], xa, dm[1], xb);
+    v0 = fmaf(down, quad_sum(r0), v0), v1 = fmaf(down, quad_sum(r1), v1);
 }
 
 template <uint32_t BYTES>
@@ -119,17 +108,7 @@ __device__ inline void fetch_record(uint8_t *dst, const uint8_t *src, uint32_t l
     for (uint32_t off = lane * 16u; off < BYTES; off += 512u) cp_async16(dst + off, src + off);
 }
 
-__device__ inline void load8(const float *src, float (&v)[8]) {
-    const float4 a = reinterpret_cast<const float4 *>(src)[0], b = reinterpret_cast<const float4 *>(src)[1];
-    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-}
-
-__device__ inline float quad_sum(float v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    return v + __shfl_xor_sync(0xffffffffu, v, 2);
-}
-
-// How the warps of a CTA share a matrix: `width` warps a row tile (a team), `records` super-blocks each.
+// How the warps of a CTA share a matrix: `width` warps a row tile (a team), `records` super-blocks each, as Members.
 struct Teams {
     uint32_t supers, row_tiles, rows, width, records, teams;
 };
@@ -168,17 +147,15 @@ __global__ void __launch_bounds__(kMaxWarps * 32) token_q8_kernel(const TokenQ8P
         load8(p.x + s * 256u + lane * 8u, v);
         if (p.norm) {
             if (r) load8(p.norm + s * 256u + lane * 8u, w);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) square = fmaf(v[i], v[i], square), v[i] *= w[i];
+            weigh8(v, w, square);
         }
-        const float unscale = stage_slice(v, lines, lane, xa, xb);
+        const float down = stage_slice(v, lines, lane, xa, xb);
         if (r == 0) {
             cp_async_wait<0>();
             __syncwarp();
         }
-        q8_record(stage + r * kB8SuperBytes, lines, unscale, lane, v0, v1);
+        q8_record(stage + r * kB8SuperBytes, lines, down, lane, v0, v1);
     }
-    v0 = quad_sum(v0), v1 = quad_sum(v1);
     if (p.norm) square = warp_sum(square);
     if ((lane & 3u) == 0) rows[warp][lane >> 2] = v0, rows[warp][(lane >> 2) + 8u] = v1;
     if (lane == 0) squares[warp] = square;
@@ -187,35 +164,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32) token_q8_kernel(const TokenQ8P
     if (!writes) return;
     float sum = 0.0f, total = 0.0f;
     for (uint32_t m = 0; m < W; ++m) sum += rows[warp + m][lane], total += squares[warp + m];
-    if (p.norm) sum *= 1.0f / sqrtf(total / (float)(p.at.supers * 256u) + p.eps);
+    if (p.norm) sum = __fmul_rn(sum, norm_scale(total, p.at.supers * 256u, p.eps));
     p.out[row] = p.residual ? add + sum : sum;
 }
 
-// One 128-wide head by one warp: lane L holds elements L, 32 + L, 64 + L, 96 + L, so both halves of a rotation pair sit in one
-// lane, and the sums are formed in the order of moe_heads_kernel's four warps: the same bits.
-__device__ inline void prepare_head(const float (&v)[4], const float (&norm)[4], const float (&cs)[2], const float (&sn)[2],
-                                    float eps, float (&out)[4]) {
-    float sum = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float s = v[k] * v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        sum += s;
-    }
-    const float scale = 1.0f / sqrtf(sum / (float)kDim + eps);
-    float head[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) head[k] = v[k] * scale * norm[k];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const float a = head[k], b = head[k + 2];
-        out[k] = a * cs[k] - b * sn[k];
-        out[k + 2] = a * sn[k] + b * cs[k];
-    }
-}
-
-constexpr uint32_t kTokenAttnWarps = 8;
+constexpr uint32_t kTokenAttnWarps = kStrands;  // a strand a warp
 
 // One CTA per KV head and span; the G query heads of the group are scored against each row once it is read.  Rows that the
 // cache held before this token, the angles and the norms are fetched before the wait.
@@ -232,7 +185,7 @@ __global__ void __launch_bounds__(kTokenAttnWarps * 32, 2) token_attention_kerne
     pdl_launch_dependents();
     const uint32_t kvh = blockIdx.x, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t position = min(*position_word, context - 1u), rows = position + 1u;  // written between tokens only
-    const uint32_t span = token_span(rows, splits), lo = split * span;
+    const uint32_t span = span_rows(rows, splits), lo = split * span;
     if (lo >= rows) return;  // the first span of every head stays
     const uint32_t hi = min(rows, lo + span);
     const size_t kv_row = (size_t)kv_heads * kDim;
@@ -251,11 +204,7 @@ __global__ void __launch_bounds__(kTokenAttnWarps * 32, 2) token_attention_kerne
     if (raw) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) qn[k] = q_norm[32 * k + lane], kn[k] = k_norm[32 * k + lane];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float angle = (float)position * powf(theta, -((float)(2u * (32u * k + lane))) / (float)kDim);
-            sincosf(angle, &sn[k], &cs[k]);
-        }
+        head_angles(position, theta, lane, cs, sn);
     }
     pdl_wait();
     if (raw) {
@@ -309,7 +258,7 @@ __global__ void __launch_bounds__(kTokenAttnWarps * 32, 2) token_attention_kerne
         for (uint32_t j = 0; j < 2u; ++j)
 #pragma unroll
             for (int g = 0; g < G; ++g)
-                dot[j][g] = qv[g].x * kv[j].x + qv[g].y * kv[j].y + qv[g].z * kv[j].z + qv[g].w * kv[j].w;
+                dot[j][g] = dot4(qv[g], kv[j]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -321,15 +270,9 @@ __global__ void __launch_bounds__(kTokenAttnWarps * 32, 2) token_attention_kerne
             if (t0 + j * kTokenAttnWarps >= hi) break;
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-                const float s = dot[j][g] * scale;
-                const float nm = fmaxf(m[g], s);
-                const float c = expf(m[g] - nm), e = expf(s - nm);
-                l[g] = l[g] * c + e;
-                acc[g].x = acc[g].x * c + e * vv[j].x;
-                acc[g].y = acc[g].y * c + e * vv[j].y;
-                acc[g].z = acc[g].z * c + e * vv[j].z;
-                acc[g].w = acc[g].w * c + e * vv[j].w;
-                m[g] = nm;
+                float c, e;
+                strand_step(m[g], l[g], __fmul_rn(dot[j][g], scale), c, e);
+                strand_add(acc[g], c, e, vv[j]);
             }
         }
     }
@@ -346,12 +289,7 @@ __global__ void __launch_bounds__(kTokenAttnWarps * 32, 2) token_attention_kerne
     float gl = 0.0f;
     float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (uint32_t w = 0; w < kTokenAttnWarps; ++w) {
-        const float c = sm[w][warp] == -INFINITY ? 0.0f : expf(sm[w][warp] - gm);
-        const float4 v = sacc[w][warp][lane];
-        gl += sl[w][warp] * c;
-        a.x += v.x * c, a.y += v.y * c, a.z += v.z * c, a.w += v.w * c;
-    }
+    for (uint32_t w = 0; w < kTokenAttnWarps; ++w) strand_take(gl, a, strand_weight(sm[w][warp], gm), sl[w][warp], sacc[w][warp][lane]);
     float *dst = part + (((size_t)kvh * G + warp) * splits + split) * (kDim + 2u);
     if (lane == 0) dst[0] = gm, dst[1] = gl;
     reinterpret_cast<float2 *>(dst + 2)[lane * 2u] = make_float2(a.x, a.y);
@@ -363,7 +301,7 @@ __global__ void __launch_bounds__(kDim) token_merge_kernel(const uint32_t *posit
                                                            uint32_t splits, uint32_t context) {
     pdl_launch_dependents();
     const uint32_t h = blockIdx.x, i = threadIdx.x, lane = i & 31u;
-    const uint32_t rows = min(*position_word, context - 1u) + 1u, span = token_span(rows, splits);
+    const uint32_t rows = min(*position_word, context - 1u) + 1u, span = span_rows(rows, splits);
     const uint32_t used = (rows + span - 1u) / span;
     const float *src = part + (size_t)h * splits * (kDim + 2u);
     pdl_wait();
@@ -374,56 +312,45 @@ __global__ void __launch_bounds__(kDim) token_merge_kernel(const uint32_t *posit
         m[j] = s < used ? src[s * (kDim + 2u)] : -INFINITY;
         l[j] = s < used ? src[s * (kDim + 2u) + 1u] : 0.0f;
     }
-    const float top = warp_max(fmaxf(m[0], m[1]));
     float c[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) c[j] = m[j] == -INFINITY ? 0.0f : expf(m[j] - top);
-    const float total = warp_sum(l[0] * c[0] + l[1] * c[1]);
+    const float total = span_weights(m, l, c);
     float a = 0.0f;
 #pragma unroll 8
     for (uint32_t s = 0; s < used; ++s) {
         const float weight = __shfl_sync(0xffffffffu, s < 32u ? c[0] : c[1], s & 31u);
-        a += src[s * (kDim + 2u) + 2u + i] * weight;
+        a = fmaf(src[s * (kDim + 2u) + 2u + i], weight, a);
     }
     out[(size_t)h * kDim + i] = a / total;
 }
 
-// One CTA per expert; its router row times the norm's weights is ready before the wait.
-constexpr uint32_t kRouterThreads = 256;
-__global__ void __launch_bounds__(kRouterThreads) token_router_kernel(const float *router, const float *x, const float *norm,
-                                                                      float eps, float *scores, uint32_t hidden) {
-    __shared__ float part[2][kRouterThreads / 32];
+// One CTA per expert, a warp a member; its router row times the norm's weights is ready before the wait.
+__global__ void __launch_bounds__(kMaxWarps * 32) token_router_kernel(const float *router, const float *x, const float *norm,
+                                                                      float eps, float *scores, const Members at) {
+    __shared__ float part[2][kMaxWarps];
     pdl_launch_dependents();
-    const float4 *row = reinterpret_cast<const float4 *>(router + (size_t)blockIdx.x * hidden);
-    const float4 *weights = reinterpret_cast<const float4 *>(norm), *in = reinterpret_cast<const float4 *>(x);
-    const auto product = [&](uint32_t i) {
-        const float4 a = row[i], b = weights[i];
-        return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
-    };
-    const uint32_t count = hidden / 4u;
-    float4 ready[2] = {};
+    const uint32_t lane = threadIdx.x & 31u, member = threadIdx.x >> 5;
+    const float *row = router + (size_t)blockIdx.x * at.supers * kSlice;
+    float a[8], w[8], v[8], dot = 0.0f, square = 0.0f;
+    const auto product = [&](uint32_t s) {
+        load8(row + s * kSlice + lane * 8u, a), load8(norm + s * kSlice + lane * 8u, w);
 #pragma unroll
-    for (uint32_t j = 0; j < 2u; ++j)
-        if (threadIdx.x + j * kRouterThreads < count) ready[j] = product(threadIdx.x + j * kRouterThreads);
+        for (int i = 0; i < 8; ++i) a[i] = __fmul_rn(a[i], w[i]);
+    };
+    product(member);
     pdl_wait();
-    float dot = 0.0f, square = 0.0f;
-    const auto add = [&](const float4 &a, uint32_t i) {
-        const float4 v = in[i];
-        dot += a.x * v.x + a.y * v.y + a.z * v.z + a.w * v.w;
-        square += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    };
+    for (uint32_t r = 0, s = member; r < at.records && s < at.supers; ++r, s += at.width) {
+        if (r) product(s);
+        load8(x + s * kSlice + lane * 8u, v);
 #pragma unroll
-    for (uint32_t j = 0; j < 2u; ++j)
-        if (threadIdx.x + j * kRouterThreads < count) add(ready[j], threadIdx.x + j * kRouterThreads);
-    for (uint32_t i = threadIdx.x + 2u * kRouterThreads; i < count; i += kRouterThreads) add(product(i), i);
+        for (int i = 0; i < 8; ++i) dot = fmaf(a[i], v[i], dot), square = fmaf(v[i], v[i], square);
+    }
     dot = warp_sum(dot), square = warp_sum(square);
-    if ((threadIdx.x & 31u) == 0) part[0][threadIdx.x >> 5] = dot, part[1][threadIdx.x >> 5] = square;
+    if (lane == 0) part[0][member] = dot, part[1][member] = square;
     __syncthreads();
     if (threadIdx.x) return;
     dot = square = 0.0f;
-#pragma unroll
-    for (uint32_t w = 0; w < kRouterThreads / 32u; ++w) dot += part[0][w], square += part[1][w];
-    scores[blockIdx.x] = dot * (1.0f / sqrtf(square / (float)hidden + eps));
+    for (uint32_t m = 0; m < at.width; ++m) dot += part[0][m], square += part[1][m];
+    scores[blockIdx.x] = __fmul_rn(dot, norm_scale(square, at.supers * kSlice, eps));
 }
 
 struct TokenGateUpParams {
@@ -499,17 +426,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 1) token_gate_up_
     for (uint32_t r = 0, s = member; r < p.at.records && s < p.at.supers; ++r, s += W) {
         float xa, xb;
         if (r) load8(p.norm + s * 256u + lane * 8u, w), load8(p.x + s * 256u + lane * 8u, v);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) square = fmaf(v[i], v[i], square), v[i] *= w[i];
-        const float unscale = stage_slice(v, lines, lane, xa, xb);
+        weigh8(v, w, square);
+        const float down = stage_slice(v, lines, lane, xa, xb);
         if (r == 0) {
             cp_async_wait<0>();
             __syncwarp();
         }
-        q4_record(stage + 2u * r * kQ4SuperBytes, lines, unscale, xa, xb, lane, g0, g1);
-        q4_record(stage + (2u * r + 1u) * kQ4SuperBytes, lines, unscale, xa, xb, lane, u0, u1);
+        q4_record(stage + 2u * r * kQ4SuperBytes, lines, down, xa, xb, lane, g0, g1);
+        q4_record(stage + (2u * r + 1u) * kQ4SuperBytes, lines, down, xa, xb, lane, u0, u1);
     }
-    g0 = quad_sum(g0), g1 = quad_sum(g1), u0 = quad_sum(u0), u1 = quad_sum(u1), square = warp_sum(square);
+    square = warp_sum(square);
     if ((lane & 3u) == 0) {
         const uint32_t g = lane >> 2;
         rows[warp][g] = g0, rows[warp][g + 8u] = g1, rows[warp][g + 16u] = u0, rows[warp][g + 24u] = u1;
@@ -520,17 +446,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 1) token_gate_up_
     if (member) return;
     float sum = 0.0f, total = 0.0f;
     for (uint32_t m = 0; m < W; ++m) sum += rows[warp + m][lane], total += squares[warp + m];
-    sum *= 1.0f / sqrtf(total / (float)(p.at.supers * 256u) + p.eps);
+    sum = __fmul_rn(sum, norm_scale(total, p.at.supers * 256u, p.eps));
     const float other = __shfl_down_sync(0xffffffffu, sum, 16);  // lanes 0-15: gate rows, 16-31: up rows
     if (lane >= 16u || tile * 16u + lane >= p.at.rows) return;
-    float sigmoid;  // two branches (engine/hybrid/math.rs:5-16)
-    if (sum >= 0.0f) {
-        sigmoid = 1.0f / (1.0f + expf(-sum));
-    } else {
-        const float e = expf(sum);
-        sigmoid = e / (1.0f + e);
-    }
-    p.act[(size_t)slot * p.at.rows + tile * 16u + lane] = sum * sigmoid * other;
+    p.act[(size_t)slot * p.at.rows + tile * 16u + lane] = gated_value(sum, other);
 }
 
 struct TokenDownParams {
@@ -574,14 +493,13 @@ __global__ void __launch_bounds__(kMaxWarps * 32) token_down_kernel(const TokenD
     for (uint32_t r = 0, s = member; r < p.at.records && s < p.at.supers; ++r, s += W) {
         float v[8], xa, xb;
         load8(p.x + ((size_t)slot * p.at.supers + s) * 256u + lane * 8u, v);
-        const float unscale = stage_slice(v, lines, lane, xa, xb);
+        const float down = stage_slice(v, lines, lane, xa, xb);
         if (r == 0) {
             cp_async_wait<0>();
             __syncwarp();
         }
-        q4_record(stage + r * kQ4SuperBytes, lines, unscale, xa, xb, lane, v0, v1);
+        q4_record(stage + r * kQ4SuperBytes, lines, down, xa, xb, lane, v0, v1);
     }
-    v0 = quad_sum(v0), v1 = quad_sum(v1);
     if ((lane & 3u) == 0) rows[warp][lane >> 2] = v0, rows[warp][(lane >> 2) + 8u] = v1;
     if (W > 1u) named_bar_sync(1 + (int)team, (int)W * 32);
     else __syncwarp();
@@ -602,37 +520,20 @@ __global__ void __launch_bounds__(kMixThreads) token_mix_kernel(float *x, const 
     float r = 0.0f;
     if (probs) {
 #pragma unroll 8
-        for (uint32_t e = 0; e < active; ++e) r += probs[e] * rows[(size_t)e * hidden + i];
+        for (uint32_t e = 0; e < active; ++e) r = fmaf(probs[e], rows[(size_t)e * hidden + i], r);
     } else {
         r = rows[i];
     }
     x[i] = before + r;
 }
 
-template <typename... Params, typename... Args>
-stark_b200_status launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, bool pdl, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    SB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
-    return STARK_B200_OK;
-}
-
 // A warp a super-block up to 16 of them; `warps` per CTA (16 where one team needs more).
 Teams teams_of(const QMatrix *w, uint32_t warps) {
     Teams at{};
-    at.supers = w->columns / 256u;
+    const Members m = members_of(w->columns);
+    at.supers = m.supers, at.width = m.width, at.records = m.records;
     at.row_tiles = w->row_tiles;
     at.rows = w->rows;
-    at.records = (at.supers + kMaxWarps - 1u) / kMaxWarps;
-    at.width = (at.supers + at.records - 1u) / at.records;
     at.teams = std::max(1u, warps / at.width);
     return at;
 }
@@ -662,7 +563,7 @@ stark_b200_status token_q8_launch(const QMatrix *w, const float *x, const float 
     static SmemOptIn once;
     if (stark_b200_status s = ensure_dynamic_smem(token_q8_kernel, kTokenSmem, once)) return s;
     const TokenQ8Params p{teams_of(w, kQ8Warps), w->data, x, norm, residual, eps, out};
-    return launch(token_q8_kernel, teams_grid(p.at, 1), p.at.teams * p.at.width * 32u, teams_smem(p.at, kB8SuperBytes), pdl, stream, p);
+    return moe_launch(token_q8_kernel, teams_grid(p.at, 1), p.at.teams * p.at.width * 32u, teams_smem(p.at, kB8SuperBytes), pdl, stream, p);
 }
 
 stark_b200_status token_attention_launch(const uint32_t *position, const float *qkv, bool raw, float *keys, float *values,
@@ -671,19 +572,20 @@ stark_b200_status token_attention_launch(const uint32_t *position, const float *
                                          cudaStream_t stream) {
     const uint32_t group = q_heads / kv_heads;
     const auto kernel = group == 8u ? token_attention_kernel<8> : (group == 4u ? token_attention_kernel<4> : token_attention_kernel<2>);
-    return launch(kernel, dim3(kv_heads, splits), kTokenAttnWarps * 32u, 0, pdl, stream, position, qkv, raw, keys, values, part,
+    return moe_launch(kernel, dim3(kv_heads, splits), kTokenAttnWarps * 32u, 0, pdl, stream, position, qkv, raw, keys, values, part,
                   splits, kv_heads, 1.0f / sqrtf((float)kDim), context, q_norm, k_norm, eps, theta);
 }
 
 stark_b200_status token_merge_launch(const uint32_t *position, const float *part, float *out, uint32_t splits, uint32_t q_heads,
                                      uint32_t context, bool pdl, cudaStream_t stream) {
     if (splits > 64u) return STARK_B200_INVALID_ARGUMENT;  // two spans a lane
-    return launch(token_merge_kernel, q_heads, kDim, 0, pdl, stream, position, part, out, splits, context);
+    return moe_launch(token_merge_kernel, q_heads, kDim, 0, pdl, stream, position, part, out, splits, context);
 }
 
 stark_b200_status token_router_launch(const float *router, const float *x, const float *norm, float eps, float *scores,
                                       uint32_t hidden, uint32_t experts, bool pdl, cudaStream_t stream) {
-    return launch(token_router_kernel, experts, kRouterThreads, 0, pdl, stream, router, x, norm, eps, scores, hidden);
+    const Members at = members_of(hidden);
+    return moe_launch(token_router_kernel, experts, at.width * 32u, 0, pdl, stream, router, x, norm, eps, scores, at);
 }
 
 stark_b200_status token_gate_up_launch(const QMatrix *w, const TokenSelection &sel, const float *x, const float *norm, float eps,
@@ -695,7 +597,7 @@ stark_b200_status token_gate_up_launch(const QMatrix *w, const TokenSelection &s
     static SmemOptIn once[4];
     if (stark_b200_status s = ensure_dynamic_smem(kernels[slot], kTokenSmem, once[slot])) return s;
     const TokenGateUpParams p{at, sel, w->data, (size_t)at.row_tiles * at.supers * kQ4SuperBytes, x, norm, eps, act};
-    return launch(kernels[slot], teams_grid(at, sel.active), at.teams * at.width * 32u, teams_smem(at, 2u * kQ4SuperBytes), pdl, stream, p);
+    return moe_launch(kernels[slot], teams_grid(at, sel.active), at.teams * at.width * 32u, teams_smem(at, 2u * kQ4SuperBytes), pdl, stream, p);
 }
 
 stark_b200_status token_down_launch(const QMatrix *w, const uint32_t *ids, uint32_t active, const float *act, float *out, bool pdl,
@@ -704,12 +606,12 @@ stark_b200_status token_down_launch(const QMatrix *w, const uint32_t *ids, uint3
     if (stark_b200_status s = ensure_dynamic_smem(token_down_kernel, kTokenSmem, once)) return s;
     const Teams at = teams_of(w, kDownWarps);
     const TokenDownParams p{at, w->data, (size_t)at.row_tiles * at.supers * kQ4SuperBytes, ids, w->experts ? w->experts : 1u, act, out};
-    return launch(token_down_kernel, teams_grid(at, active), at.teams * at.width * 32u, teams_smem(at, kQ4SuperBytes), pdl, stream, p);
+    return moe_launch(token_down_kernel, teams_grid(at, active), at.teams * at.width * 32u, teams_smem(at, kQ4SuperBytes), pdl, stream, p);
 }
 
 stark_b200_status token_mix_launch(float *x, const float *rows, const float *probs, uint32_t active, uint32_t hidden, bool pdl,
                                    cudaStream_t stream) {
-    return launch(token_mix_kernel, (hidden + kMixThreads - 1u) / kMixThreads, kMixThreads, 0, pdl, stream, x, rows, probs, active,
+    return moe_launch(token_mix_kernel, (hidden + kMixThreads - 1u) / kMixThreads, kMixThreads, 0, pdl, stream, x, rows, probs, active,
                   hidden);
 }
 

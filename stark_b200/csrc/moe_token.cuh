@@ -5,13 +5,6 @@
 namespace sb {
 
 constexpr uint32_t kEpSkip = 0xffffffffu;  // expert id of a selection slot another rank owns
-constexpr uint32_t kTokenMinSpan = 16;     // cache rows a CTA of the token's attention takes at least: two for every warp
-
-// Cache rows per span, and with it the spans that hold any, of a token that sees `rows` rows.
-__host__ __device__ inline uint32_t token_span(uint32_t rows, uint32_t splits) {
-    const uint32_t even = (rows + splits - 1u) / splits;
-    return even > kTokenMinSpan ? even : kTokenMinSpan;
-}
 
 // Whether the token kernels take these matrices: formats of 16 x 256 records, rows that fit the warps of a CTA.
 bool token_q8_supports(const QMatrix *w);

@@ -75,8 +75,7 @@ def _rank_main(config: str) -> None:
     if rank == 0:
         # one GPU, same weights: the exchange must not change a bit
         single = MoEModel.load(cfg, w, context)
-        for t in prompt[:-1]:                               # a token at a time, as ranks do: a pass of rows sums in another order
-            single.ingest([t])
+        single.ingest(prompt[:-1])
         want = single.step(int(prompt[-1]))
         assert np.array_equal(single.last_experts(), experts)
         assert np.array_equal(want.view(np.uint32), logits.view(np.uint32))
@@ -94,8 +93,7 @@ def _rank_main(config: str) -> None:
     again = model.step(int(prompt[5]))
     if rank == 0:
         single = MoEModel.load(cfg, w, context)
-        for t in prompt[:5]:
-            single.ingest([t])
+        single.ingest(prompt[:5])
         assert np.array_equal(single.step(int(prompt[5])).view(np.uint32), again.view(np.uint32))
         single.close()
     model.close()

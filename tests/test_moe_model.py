@@ -225,11 +225,40 @@ def test_prompt_rows_in_passes(name, portions):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("sizes,portions", [
+    (dict(), (2, 15, 16, 17, 3, 515)),                                                                     # passes of every raggedness
+    (dict(hidden=2048, q_heads=32, kv_heads=4, experts=128, active=8, inter=768), (33, 260)),             # spans of 16 rows and more
+    (dict(hidden=4352, inter=4864, experts=5, active=3, q_heads=34, kv_heads=17), (18,)),                 # rows of more slices than warps
+    (dict(hidden=8192, inter=256, experts=300, active=32, q_heads=8, kv_heads=1), (5, 40)),               # the widest; most picks
+    (dict(hidden=768, inter=512, experts=129, active=1, q_heads=10, kv_heads=5), (17, 1020))])
+def test_rows_of_a_pass_leave_a_tokens_bits(sizes, portions):
+    """A prompt in portions, and its rows one by one (as ranks of a group take them): the same logits, experts and tokens."""
+    from stark_b200.engine import MoEModel
+    cfg = dict(S.MOE_CONFIGS["moe-tiny"], **sizes)
+    w = S.moe_weights(cfg, seed=21)
+    context = sum(portions) + 8
+    ids = S.prompt(cfg, context, seed=31)
+    seen = []
+    for single in (False, True):
+        model, at, out = MoEModel.load(cfg, w, context), 0, []
+        for n in portions:
+            for part in ([ids[i:i + 1] for i in range(at, at + n)] if single else [ids[at:at + n]]):
+                model.ingest(part)
+            at += n
+            out.append(model.last_experts().tobytes())
+        out += [model.step(int(ids[at])).tobytes(), model.last_experts().tobytes(), model.generate_greedy(int(ids[at + 1]), 4).tobytes()]
+        seen.append(out)
+        model.close()
+    assert seen[0] == seen[1]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("sizes", [
-    dict(hidden=12288), dict(hidden=12544), dict(q_heads=96, kv_heads=12), dict(q_heads=98, kv_heads=49), dict(inter=12288), dict(inter=12544)])
+    dict(hidden=8192), dict(hidden=8448), dict(hidden=12288), dict(hidden=12544), dict(q_heads=96, kv_heads=12), dict(q_heads=98, kv_heads=49),
+    dict(inter=12288), dict(inter=12544)])
 def test_prompt_rows_of_the_widest_models(sizes):
     """Row widths at the most that a pass of rows takes and one step past it: rows go one by one then, and input rows of q, k, v
-    and o past the matvec's own bound are refused."""
+    and o past the matvec's own bound are refused.  12 288 columns are the 48 KB of shared memory a launch has unasked."""
     from stark_b200._lib import StarkB200Error
     from stark_b200.engine import MoEModel
     cfg = dict(S.MOE_CONFIGS["moe-tiny"], layers=2, experts=4, active=2, **sizes)
