@@ -24,8 +24,7 @@ constexpr uint32_t kMostRecords = 8;  // of a warp's slice: two 16-byte chunks o
 struct ShortParams {
     const uint8_t *w;
     uint32_t rows, groups, pair_halves, slice;  // slice: records of a warp's columns in shared memory
-    const uint16_t *x, *norm_bf16, *resid;
-    const float *norm;
+    const uint16_t *x, *norm, *resid;
     float eps;
     uint32_t epilogue;
     uint16_t *y;
@@ -60,13 +59,7 @@ __global__ void __launch_bounds__(kThreads) qmv_a4_short_kernel(const ShortParam
         for (uint32_t r = 0; r < 2u; ++r) {
             const uint32_t c = lane + 32u * r;
             if (c >= count * 8u) continue;
-            if (p.norm_bf16) {
-                nw[r] = reinterpret_cast<const uint4 *>(p.norm_bf16 + first * 64u)[c];
-            } else {
-                const float4 *n4 = reinterpret_cast<const float4 *>(p.norm + first * 64u) + 2u * c;
-                const float4 a = n4[0], b = n4[1];
-                nw[r] = make_uint4(f32x2_to_bf16x2(a.x, a.y), f32x2_to_bf16x2(a.z, a.w), f32x2_to_bf16x2(b.x, b.y), f32x2_to_bf16x2(b.z, b.w));
-            }
+            nw[r] = reinterpret_cast<const uint4 *>(p.norm + first * 64u)[c];
         }
     pdl_wait();
     const uint32_t row = tile_row0(tile0, p.pair_halves, p.rows) + lane;  // what this lane of warp 0 stores
@@ -201,7 +194,7 @@ bool qmv_short_takes(const QmvArgs &a) {
     if (!tunables().qmv_short || a.io_type != STARK_B200_BF16 || a.exchange || a.trace || m->bytes > kShortBytes ||
         m->groups > kWarps * kMostRecords)
         return false;
-    if (a.prologue != kProPlain && a.prologue != kProRmsNorm) return false;
+    if (a.prologue != kProPlain && !(a.prologue == kProRmsNorm && a.norm_weight_bf16)) return false;
     if (!pair && a.epilogue != kEpiStore && a.epilogue != kEpiResidual) return false;
     if (pair && m->row_tiles % 2u) return false;
     const uint32_t each = (m->row_tiles / (pair ? 2u : 1u) + 147u) / 148u;
@@ -219,7 +212,7 @@ stark_b200_status qmv_short_launch(const QmvArgs &a, cudaStream_t stream) {
     if (stark_b200_status s = ensure_dynamic_smem(kernels[slot], 150 * 1024, once[slot])) return s;
     if (a.out_grid) *a.out_grid = grid;
     const ShortParams p{m->data, m->rows, m->groups, m->pair_halves, short_slice(m), static_cast<const uint16_t *>(a.x), a.norm_weight_bf16,
-                        static_cast<const uint16_t *>(a.resid), a.norm_weight, a.eps, a.epilogue, static_cast<uint16_t *>(a.y)};
+                        static_cast<const uint16_t *>(a.resid), a.eps, a.epilogue, static_cast<uint16_t *>(a.y)};
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThreads);

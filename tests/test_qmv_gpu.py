@@ -54,15 +54,44 @@ def test_matrices_requested_whole(rows, columns):
     make = lambda pair: QMatrix.from_affine(w["codes"], w["scales"], w["biases"], rows, columns, pair_halves=pair)  # noqa: E731
     plain, pair = make(False), make(True) if rows % 32 == 0 else None
     seen = []
-    for short in (0, 1):
-        _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", short), "set_tunable")
-        seen.append((plain.matvec(w["x"]), qmv_swiglu(pair, w["x"]) if pair else None))
+    try:
+        for short in (0, 1):
+            _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", short), "set_tunable")
+            seen.append((plain.matvec(w["x"]), qmv_swiglu(pair, w["x"]) if pair else None))
+    finally:
+        _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", 1), "set_tunable")
     assert take_device_error() == 0
     for streamed, whole in zip(*seen):
         if streamed is None:
             continue
         assert (streamed != whole).mean() < 0.02
         assert _rel_err(whole, streamed).max() <= 3 * 2.0 ** -7  # a unit of the last place; of both factors and their product
+
+
+@pytest.mark.parametrize("hidden,inter", [(64, 64), (192, 448), (576, 64), (1024, 1216), (4096, 320)])
+def test_matrices_requested_whole_with_norm_and_residual(hidden, inter):
+    """The forms that only a token uses -- the norm in the prologue (fewer column groups than warps, ragged slices, the widest
+    row), the residual in the epilogue -- through one layer, against the streaming kernel and the oracle."""
+    from stark_b200 import _lib
+    from stark_b200.engine import DenseModel
+    from stark_b200.ops import take_device_error
+    from tests.test_model_gpu import assert_logits_accepted
+    cfg = dict(S.CONFIGS["tiny"], layers=1, hidden=hidden, inter=inter, q_heads=2, kv_heads=1, vocab=512)
+    w = S.dense_weights(cfg, seed=hidden, zero_point=7.5)
+    ids, seen = S.prompt(cfg, 3, seed=4), []
+    try:
+        for short in (0, 1):
+            _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", short), "set_tunable")
+            model = DenseModel.load(cfg, w, context_tokens=16)
+            seen.append([O.f32_to_bf16(model.step(int(t))) for t in ids])
+            model.close()
+    finally:
+        _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", 1), "set_tunable")
+    assert take_device_error() == 0
+    oracle = O.DenseOracle(cfg, w, capacity=16)
+    for t, streamed, whole in zip(ids, *seen):
+        assert_logits_accepted(streamed, whole)
+        assert_logits_accepted(oracle.step(int(t)), whole)
 
 
 def test_matvec_group_output_plane_layout():
