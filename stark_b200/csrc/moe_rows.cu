@@ -10,6 +10,8 @@
 //
 // Every sum over a row, a slice of 256 columns, a strand of keys or the spans is formed as a token forms it (moe_math.cuh): a
 // row's results are the token's, bit for bit.
+//
+// 12 layers of the 30B-A3B shape, 160 rows and the token behind them: 4.56 ms against 112 ms token by token.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -53,8 +55,8 @@ __device__ inline uint32_t slice_at(const Members &at, uint32_t step, bool &ends
 }
 
 // One CTA: 16 matrix rows a warp times up to 16 input rows, the contraction in steps of 256 columns, copies of the
-// next steps in flight.  Bound by issue slots of the tensor-core loop at full tiles (10 instructions per two products) and by
-// the weights' bytes where experts have few rows.
+// next steps in flight.  Bound by the latency of the tensor-core loop at full tiles, 16 warps an SM at 128 registers, and by the
+// weights' bytes where experts have few rows.  160 rows, 8 of 128 experts: gate and up 151 us, down 82.
 // MULTI: members of several slices.
 template <bool Q4, int STAGES, uint32_t WARPS, bool MULTI>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8u && !MULTI ? 2 : 1) rows_gemm_kernel(const RowsGemmParams p) {
@@ -335,14 +337,21 @@ __device__ inline float group_sums(float (&d)[G], uint32_t lane) {
 constexpr uint32_t kSpanState = kHeadWidth + 4u;
 
 // Attention of a row, `each` spans of a KV head a CTA: as in a token a warp is a strand, which reads a key once for the G query
-// heads of the group; 32 / G lanes keep the maximum and sum of a head.  Bound by instruction issue.
+// heads of the group; 32 / G lanes keep the maximum and sum of a head.  Two keys of a strand go side by side up to their
+// scores, and the next two are fetched meanwhile.  A span's strands merge through one of two buffers, so that a barrier a span
+// is enough.  Bound by instruction issue and that barrier: 160 rows of 32 heads behind 500 take 201 us, 209 with one key at a time
+// and one buffer, 238 with a warp a query head, 350 with every lane computing every weight.
+template <int G>
+struct SpanBuffer {
+    float m[kStrands][G], l[kStrands][G];
+    float4 acc[kStrands][G][32];
+};
 template <int G>
 __global__ void __launch_bounds__(kStrands * 32, 2) moe_rows_attention_kernel(const float *qkv, const float *keys, const float *values,
                                                                               float *part, uint32_t first_pos, uint32_t splits,
                                                                               uint32_t each, uint32_t spans, uint32_t kv_heads, float scale) {
     constexpr uint32_t kLanes = 32u / G;
-    __shared__ float sm[kStrands][G], sl[kStrands][G];
-    __shared__ __align__(16) float4 sacc[kStrands][G][32];
+    extern __shared__ __align__(16) uint8_t span_smem[];
     const uint32_t kvh = blockIdx.x, row = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t rows = first_pos + row + 1u, span = span_rows(rows, splits), used = (rows + span - 1u) / span;
     const uint32_t from = blockIdx.y * each, to = min(used, from + each);
@@ -357,36 +366,53 @@ __global__ void __launch_bounds__(kStrands * 32, 2) moe_rows_attention_kernel(co
 #pragma unroll
     for (int g = 0; g < G; ++g)
         q[g] = reinterpret_cast<const float4 *>(qkv + ((size_t)row * kv_heads * (G + 2u) + kvh * G + g) * kHeadWidth)[lane];
-    float4 k = fetch(keys, from * span + warp), v = fetch(values, from * span + warp);
+    float4 k[2], v[2];
+#pragma unroll
+    for (uint32_t j = 0; j < 2u; ++j) {
+        const uint32_t t = from * span + warp + j * kStrands;
+        k[j] = fetch(keys, t), v[j] = fetch(values, t);
+    }
     for (uint32_t n = from; n < to; ++n) {
+        SpanBuffer<G> &buffer = reinterpret_cast<SpanBuffer<G> *>(span_smem)[n & 1u];
         const uint32_t lo = n * span, hi = min(rows, lo + span);
         float m = -INFINITY, l = 0.0f;
         float4 acc[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) acc[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (uint32_t t = lo + warp; t < hi; t += kStrands) {
-            const float4 now = k, value = v;
-            const uint32_t next = t + kStrands < hi ? t + kStrands : hi + warp;  // of this span, or the first of the next
-            k = fetch(keys, next), v = fetch(values, next);
-            float dot[G], c, e;
+        for (uint32_t t = lo + warp; t < hi; t += 2u * kStrands) {
+            float score[2];
+            float4 value[2];
+            const uint32_t next = t + 2u * kStrands < hi ? t + 2u * kStrands : hi + warp;  // of this span, or the first of the next
 #pragma unroll
-            for (int g = 0; g < G; ++g) dot[g] = dot4(q[g], now);
-            strand_step(m, l, __fmul_rn(group_sums<G>(dot, lane), scale), c, e);
+            for (uint32_t j = 0; j < 2u; ++j) {
+                float dot[G];
 #pragma unroll
-            for (int g = 0; g < G; ++g) strand_add(acc[g], __shfl_sync(0xffffffffu, c, g * kLanes), __shfl_sync(0xffffffffu, e, g * kLanes), value);
+                for (int g = 0; g < G; ++g) dot[g] = dot4(q[g], k[j]);
+                value[j] = v[j];
+                k[j] = fetch(keys, next + j * kStrands), v[j] = fetch(values, next + j * kStrands);
+                score[j] = __fmul_rn(group_sums<G>(dot, lane), scale);
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 2u; ++j) {
+                if (t + j * kStrands >= hi) break;
+                float c, e;
+                strand_step(m, l, score[j], c, e);
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    strand_add(acc[g], __shfl_sync(0xffffffffu, c, g * kLanes), __shfl_sync(0xffffffffu, e, g * kLanes), value[j]);
+            }
         }
-        __syncthreads();  // the span before this one has been merged
-        if (lane % kLanes == 0) sm[warp][lane / kLanes] = m, sl[warp][lane / kLanes] = l;
+        if (lane % kLanes == 0) buffer.m[warp][lane / kLanes] = m, buffer.l[warp][lane / kLanes] = l;
 #pragma unroll
-        for (int g = 0; g < G; ++g) sacc[warp][g][lane] = acc[g];
-        __syncthreads();
+        for (int g = 0; g < G; ++g) buffer.acc[warp][g][lane] = acc[g];
+        __syncthreads();  // the span two before this one was merged ahead of the barrier between them
         if (warp >= (uint32_t)G) continue;
         float top = -INFINITY, sum = 0.0f;
 #pragma unroll
-        for (uint32_t w = 0; w < kStrands; ++w) top = fmaxf(top, sm[w][warp]);
+        for (uint32_t w = 0; w < kStrands; ++w) top = fmaxf(top, buffer.m[w][warp]);
         float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-        for (uint32_t w = 0; w < kStrands; ++w) strand_take(sum, a, strand_weight(sm[w][warp], top), sl[w][warp], sacc[w][warp][lane]);
+        for (uint32_t w = 0; w < kStrands; ++w) strand_take(sum, a, strand_weight(buffer.m[w][warp], top), buffer.l[w][warp], buffer.acc[w][warp][lane]);
         float *dst = part + (((size_t)row * kv_heads * G + kvh * G + warp) * spans + n) * kSpanState;
         if (lane == 0) *reinterpret_cast<float2 *>(dst) = make_float2(top, sum);
         reinterpret_cast<float4 *>(dst)[lane + 1u] = a;
@@ -690,11 +716,14 @@ stark_b200_status moe_rows_attention_launch(const float *qkv, const float *keys,
     const size_t row_floats = moe_rows_part(q_heads, spans);
     if (out.columns != q_heads * kHeadWidth || splits > 64u || part_floats < row_floats) return STARK_B200_INVALID_ARGUMENT;
     const auto kernel = group == 8u ? moe_rows_attention_kernel<8> : (group == 4u ? moe_rows_attention_kernel<4> : moe_rows_attention_kernel<2>);
+    const size_t smem = 2u * (group == 8u ? sizeof(SpanBuffer<8>) : (group == 4u ? sizeof(SpanBuffer<4>) : sizeof(SpanBuffer<2>)));
+    static SmemOptIn once[3];
+    if (stark_b200_status s = ensure_dynamic_smem(kernel, (int)smem, once[group / 4u])) return s;
     const uint32_t batch = (uint32_t)std::min<size_t>(rows, part_floats / row_floats);
     for (uint32_t done = 0; done < rows; done += batch) {
         const uint32_t now = std::min(batch, rows - done), pos = first_pos + done;
         const uint32_t each = std::max(1u, std::min(spans, kv_heads * spans * now / kAttentionCtas));
-        if (stark_b200_status s = launch(kernel, dim3(kv_heads, (spans + each - 1u) / each, now), kStrands * 32u, 0, stream,
+        if (stark_b200_status s = launch(kernel, dim3(kv_heads, (spans + each - 1u) / each, now), kStrands * 32u, smem, stream,
                                          qkv + (size_t)done * (q_heads + 2u * kv_heads) * kHeadWidth, keys, values, part, pos, splits, each,
                                          spans, kv_heads, 1.0f / sqrtf((float)kHeadWidth)))
             return s;
