@@ -185,8 +185,8 @@ uint32_t short_smem(const QMatrix *m, uint32_t tiles) {
 }  // namespace
 
 // One wave of CTAs whose records all fit the SMs beside a launch that waits: at most four an SM and 150 KB of them; rows of up
-// to 4 096 values (two chunks a lane).  No more than 4 MB: 4096 x 4096 (9.4 MB) takes 7.65 us against 7.47 streamed, and the
-// qkv and o projections of the 8b shape leave its token where it was.  Setting qmv_short: 0 never.
+// to 4 096 values (two chunks a lane).  No more than 4 MB: 4096 x 4096 (9.4 MB) takes 5.5 us against 4.9 streamed, twenty of
+// them in turn in a graph, and the qkv and o projections of the 8b shape leave its token where it was.  Setting qmv_short: 0 never.
 constexpr size_t kShortBytes = 4u << 20;
 bool qmv_short_takes(const QmvArgs &a) {
     const QMatrix *m = a.matrix;
