@@ -187,6 +187,9 @@ uint32_t short_smem(const QMatrix *m, uint32_t tiles) {
 // One wave of CTAs whose records all fit the SMs beside a launch that waits: at most four an SM and 150 KB of them; rows of up
 // to 4 096 values (two chunks a lane).  No more than 4 MB: 4096 x 4096 (9.4 MB) takes 5.5 us against 4.9 streamed, twenty of
 // them in turn in a graph, and the qkv and o projections of the 8b shape leave its token where it was.  Setting qmv_short: 0 never.
+// A bare row takes it with one CTA an SM at most: twenty in turn in a graph, 2368 x 1024 (148 CTAs) 2.21 -> 1.53 us, but 2560 x
+// 1024 (160) 2.51 -> 3.08 and 4096 x 1024 2.68 -> 3.27.  Behind a norm or gated, two an SM are about even: with one at most a
+// sampled answer on the 0.6b shape takes 10.9 ms (11.1), a prompt behind a prefix 2.44 (2.40).
 constexpr size_t kShortBytes = 4u << 20;
 bool qmv_short_takes(const QmvArgs &a) {
     const QMatrix *m = a.matrix;
@@ -198,6 +201,7 @@ bool qmv_short_takes(const QmvArgs &a) {
     if (!pair && a.epilogue != kEpiStore && a.epilogue != kEpiResidual) return false;
     if (pair && m->row_tiles % 2u) return false;
     const uint32_t each = (m->row_tiles / (pair ? 2u : 1u) + 147u) / 148u;
+    if (each > 1u && !pair && a.prologue == kProPlain) return false;
     return each <= 4u && each * short_smem(m, pair ? 2u : 1u) <= 150u * 1024u;
 }
 

@@ -46,8 +46,8 @@ def test_matvec_bf16_matches_oracle(rows, columns):
 
 @pytest.mark.parametrize("rows,columns", [(16, 64), (40, 192), (1000, 1024), (1760, 4096), (9472, 576), (1024, 3072), (2080, 448)])
 def test_matrices_requested_whole(rows, columns):
-    """Fewer column groups than warps, ragged slices, a last row tile in part, the widest row and the most tiles, plain and
-    gated, against the streaming kernel: the same products, f32 sums formed in another order, one rounding to bf16."""
+    """Fewer column groups than warps, ragged slices, a last row tile in part, the widest row and the most tiles, plain (up
+    to 148 tiles) and gated, against the streaming kernel: the same products, f32 sums formed in another order, one rounding to bf16."""
     from stark_b200 import _lib
     from stark_b200.ops import QMatrix, qmv_swiglu, take_device_error
     w = S.matvec_case(seed=5 + rows, rows=rows, columns=columns)
