@@ -746,6 +746,7 @@ static void dense_destroy(Model *m) {
         cudaFree(m->chunk_h);
         cudaFree(m->chunk_act);
     }
+    cudaFree(m->chunk_weights);
     cudaFree(m->chunk_x);
     cudaFree(m->chunk_qkv);
     cudaFree(m->chunk_attn);

@@ -34,10 +34,16 @@ struct GemmArgs {
     uint32_t peers = 0;
     // Output features over all ranks (0: this matrix's): the order of a sum follows from them, the same on one GPU and on several.
     uint32_t whole_rows = 0;
+    // Many rows: the weights are unpacked to bf16 rows once a pass (rmsnorm_rows_launch) and contracted from there.  may_unpack decides
+    // the tile, and with it the order of a sum; without the unpacked rows the same tile runs over the packed weights.
+    bool may_unpack = false;
+    const uint16_t *unpacked = nullptr;
 };
 constexpr uint32_t kPrefillSmallRows = 16;  // up to this many rows attend in the few-rows form
 // One launch; the kernel bounds every wait and reports through the error word.
 stark_b200_status prefill_gemm_launch(const GemmArgs &args, cudaStream_t stream);
+// Bytes of the weights as bf16 rows where the launch prefers them so, else 0.
+size_t prefill_gemm_unpacked_bytes(const GemmArgs &args);
 // Whether the launch takes the tiles that can store to peers.
 bool prefill_gemm_wide(const GemmArgs &args);
 // ---- row-wise operators over a chunk of M rows (prefill_ops.cu) ---------------------------------------
@@ -49,6 +55,10 @@ stark_b200_status embed_rows_launch(const QMatrix *table, const uint32_t *tokens
 // into a wider buffer (the [e ; h] rows of the draft head's fusion input)
 stark_b200_status rmsnorm_rows_launch(const uint16_t *h, const float *weight, uint16_t *out, uint32_t m, uint32_t d,
                                       float eps, cudaStream_t stream, uint32_t in_stride = 0, uint32_t out_stride = 0);
+// The same launch also writes up to two matrices as bf16 rows (to[i] == nullptr: that one stays packed): all of it is memory traffic, and
+// the contractions behind it read each weight once instead of dequantizing it for every 256 rows.
+stark_b200_status rmsnorm_rows_unpack_launch(const uint16_t *h, const float *weight, uint16_t *out, uint32_t m, uint32_t d, float eps,
+                                             const QMatrix *const (&w)[2], uint16_t *const (&to)[2], cudaStream_t stream);
 // first[i] = first index of the maximum of row i of a [m, n] bf16 matrix (UINT32_MAX if a value is not finite):
 // the greedy read-out of several rows at once (unified_sampling.rs:42-45, 108-113)
 stark_b200_status argmax_rows_launch(const uint16_t *rows, uint32_t m, uint32_t n, uint32_t *first, cudaStream_t stream);

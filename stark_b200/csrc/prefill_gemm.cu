@@ -23,7 +23,9 @@
 
 #include <algorithm>
 
+#include "a4_record.cuh"
 #include "device_math.cuh"
+#include "pair_gemm.cuh"
 #include "prefill.cuh"
 #include "tc05.cuh"
 #include "thin_tile.cuh"
@@ -64,75 +66,128 @@ struct GemmParams {
 // Instruction descriptor: D f32, A bf16 (activations), B bf16 (dequantized weights), both K-major, M 128, N 256.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((128u >> 4) << 24);
 
-struct RecordRegs {
-    uint4 q;
-    uint32_t scales, biases;  // bf16 pairs: rows g and g + 8
-};
-
-__device__ inline RecordRegs load_record(const uint8_t *w, uint32_t tile, uint32_t row_tiles, uint32_t groups,
-                                         uint32_t kg, uint32_t lane) {
-    RecordRegs r;
-    if (tile < row_tiles) {
-        const uint8_t *rec = w + ((size_t)tile * groups + kg) * kA4RecordBytes;
-        r.q = ldg_nc_v4(rec + lane * 16u);
-        r.scales = __ldg(reinterpret_cast<const uint32_t *>(rec + 512u + 4u * (lane >> 2)));
-        r.biases = __ldg(reinterpret_cast<const uint32_t *>(rec + 544u + 4u * (lane >> 2)));
-    } else {  // past the last row tile: zero rows
-        r.q = make_uint4(0u, 0u, 0u, 0u);
-        r.scales = 0u;
-        r.biases = 0u;
-    }
-    return r;
-}
-
-// One record word -> the eight codes as exact bf16 integers, in the fragment order of dequant_a4_word:
-// (w >> 4s) & 0x000f000f | 0x43004300 is the bf16 pair (128 + q, 128 + q') -- 0x4300 is 128.0 and the last
-// mantissa bit of a bf16 in [128, 256) weighs 1 -- and 128 is then subtracted exactly.
-__device__ inline void codes_to_bf16(uint32_t w, __nv_bfloat162 (&q)[4]) {
-    const uint32_t magic = 0x43004300u;
-    const __nv_bfloat162 k128 = __float2bfloat162_rn(128.0f);
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const uint32_t v = lop3_and_or(w >> (4 * s), 0x000f000fu, magic);
-        q[s] = __hsub2(*reinterpret_cast<const __nv_bfloat162 *>(&v), k128);
-    }
-}
-__device__ inline __nv_bfloat162 bf16_pair(uint32_t bits16) {
-    const uint32_t v = bits16 | (bits16 << 16);
-    return *reinterpret_cast<const __nv_bfloat162 *>(&v);
-}
-
-// One record (16 features x 64 columns) into rows [16 d, 16 d + 16) of the B stage: lane (g, t) owns columns
-// 16 t .. 16 t + 15 of rows g and g + 8, i.e. two 16-byte chunks in each of the two rows.
+// One record (16 features x 64 columns) into rows [16 d, 16 d + 16) of the B stage: two 16-byte chunks of a lane in each of its two rows.
 __device__ inline void dequant_record_to_smem(const RecordRegs &r, uint8_t *b_stage, uint32_t d, uint32_t lane) {
     const uint32_t g = lane >> 2, t = lane & 3u;
-    const __nv_bfloat162 s0 = bf16_pair(r.scales & 0xffffu), s1 = bf16_pair(r.scales >> 16);
-    const __nv_bfloat162 b0 = bf16_pair(r.biases & 0xffffu), b1 = bf16_pair(r.biases >> 16);
-    const uint32_t ww[4] = {r.q.x, r.q.y, r.q.z, r.q.w};
-    uint32_t lo_row[8], hi_row[8];  // 16 bf16 values per row
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        __nv_bfloat162 a[4];
-        codes_to_bf16(ww[j], a);  // a[0], a[2]: row g, columns 4j + {0,1}, {2,3}; a[1], a[3]: row g + 8
-        // bf16(scale * q + bias): one fused multiply-add, one rounding -- the dequantized operand in the
-        // activations' type, as the reference's tiled GEMM stages it (gemm.metal:122-203, `threadgroup BT b_shared`)
-        const __nv_bfloat162 v0 = __hfma2(a[0], s0, b0);
-        const __nv_bfloat162 v2 = __hfma2(a[2], s0, b0);
-        const __nv_bfloat162 v1 = __hfma2(a[1], s1, b1);
-        const __nv_bfloat162 v3 = __hfma2(a[3], s1, b1);
-        lo_row[2 * j] = *reinterpret_cast<const uint32_t *>(&v0);
-        lo_row[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&v2);
-        hi_row[2 * j] = *reinterpret_cast<const uint32_t *>(&v1);
-        hi_row[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&v3);
-    }
+    uint4 v[4];
+    dequant_record(r, v);
     // row R of the stage starts at R * 128; its 16-byte chunk c sits at chunk position c ^ (R & 7)
     const uint32_t r_lo = 16u * d + g, r_hi = r_lo + 8u;  // both have (R & 7) == g
     uint8_t *p_lo = b_stage + r_lo * 128u, *p_hi = b_stage + r_hi * 128u;
     const uint32_t c0 = ((2u * t) ^ g) * 16u, c1 = ((2u * t + 1u) ^ g) * 16u;
-    *reinterpret_cast<uint4 *>(p_lo + c0) = make_uint4(lo_row[0], lo_row[1], lo_row[2], lo_row[3]);
-    *reinterpret_cast<uint4 *>(p_lo + c1) = make_uint4(lo_row[4], lo_row[5], lo_row[6], lo_row[7]);
-    *reinterpret_cast<uint4 *>(p_hi + c0) = make_uint4(hi_row[0], hi_row[1], hi_row[2], hi_row[3]);
-    *reinterpret_cast<uint4 *>(p_hi + c1) = make_uint4(hi_row[4], hi_row[5], hi_row[6], hi_row[7]);
+    *reinterpret_cast<uint4 *>(p_lo + c0) = v[0];
+    *reinterpret_cast<uint4 *>(p_lo + c1) = v[1];
+    *reinterpret_cast<uint4 *>(p_hi + c0) = v[2];
+    *reinterpret_cast<uint4 *>(p_hi + c1) = v[3];
+}
+
+// 32 columns of a warp's 32 accumulator rows, from storage row f0 of the matrix: bf16 rounding, residual add or SwiGLU, to this rank's
+// buffer and the other ranks'.  `scratch`: the warp's own 32 rows of 80 bytes.
+__device__ __forceinline__ void store_block(const GemmParams &p, uint32_t row, uint32_t f0, const uint32_t (&acc)[32], uint8_t *scratch,
+                                            uint32_t lane, bool acc_ok) {
+    const bool row_ok = row < p.m;
+    if (p.epilogue == kEpiSwiGlu) {
+        // storage tiles alternate up / gate (pair_halves): columns 0-15 up rows, 16-31 the gate rows
+        // of the same logical rows.  gated_act_mul.rs:80-95: silu in f32 -> bf16, product -> bf16
+        uint32_t packed[8];
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            float o2[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float up = bf16_round(__uint_as_float(acc[i + e]));
+                const float gate = bf16_round(__uint_as_float(acc[16 + i + e]));
+                const float activated = bf16_round(gate / (1.0f + expf(-1.0f * gate)));
+                o2[e] = up * activated;
+            }
+            packed[i >> 1] = f32x2_to_bf16x2(o2[0], o2[1]);
+        }
+        const uint32_t o0 = (f0 / 32u) * 16u;  // logical row of the pair
+        if (row_ok && o0 + 16u <= p.rows / 2u) {
+            uint4 *dst = reinterpret_cast<uint4 *>(p.out + (size_t)row * p.ld_out + o0);
+            dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+        }
+        if (p.peers && acc_ok) {
+            // The same 32 x 16 block to the other ranks.  A lane holds 32 bytes of ITS row: stored from here, one
+            // instruction would touch 32 rows with 16 bytes each, and over NVLink every such fragment is a packet
+            // of its own.  Through the warp's scratch rows (48-byte pitch: conflict-free) the lanes regroup
+            // so that two neighbours write one row's 32 contiguous bytes.
+            uint4 *mine = reinterpret_cast<uint4 *>(scratch + lane * 48u);
+            mine[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            mine[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+            __syncwarp();
+#pragma unroll
+            for (uint32_t j = 0; j < 2u; ++j) {
+                const uint32_t r = 16u * j + (lane >> 1), q = lane & 1u;
+                const uint4 v = *reinterpret_cast<const uint4 *>(scratch + r * 48u + q * 16u);
+                const uint32_t prow = row - lane + r;
+                if (prow < p.m && o0 + 16u <= p.rows / 2u) {
+                    const size_t at = (size_t)prow * p.ld_out + o0 + q * 8u;
+#pragma unroll
+                    for (uint32_t k = 0; k + 1u < kMaxExchangeRanks; ++k) {
+                        if (k >= p.peers) break;
+                        *reinterpret_cast<uint4 *>(p.peer_out[k] + at) = v;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    } else {
+        const bool cols_ok = f0 + 32u <= p.rows;
+        uint16_t *dst16 = p.out + (size_t)row * p.ld_out + f0;
+        uint32_t packed[16];
+        if (p.epilogue == kEpiResidual && row_ok && cols_ok) {
+            const uint4 *src = reinterpret_cast<const uint4 *>(dst16);
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+                const uint4 rv = src[q4];
+                const uint32_t rr[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = q4 * 8 + e * 2;
+                    const uint32_t y2 = f32x2_to_bf16x2(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]));
+                    packed[q4 * 4 + e] = f32x2_to_bf16x2(__uint_as_float(y2 << 16) + __uint_as_float(rr[e] << 16),
+                                                         __uint_as_float(y2 & 0xffff0000u) +
+                                                             __uint_as_float(rr[e] & 0xffff0000u));
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; i += 2)
+                packed[i >> 1] = f32x2_to_bf16x2(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]));
+        }
+        if (row_ok && cols_ok) {
+            uint4 *dst = reinterpret_cast<uint4 *>(dst16);
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4)
+                dst[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
+        }
+        if (p.peers && acc_ok) {
+            // to the other ranks, regrouped through the warp's scratch rows (80-byte pitch) so that four
+            // neighbouring lanes write one row's 64 contiguous bytes (see the gated branch)
+            uint4 *mine = reinterpret_cast<uint4 *>(scratch + lane * 80u);
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4)
+                mine[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
+            __syncwarp();
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; ++j) {
+                const uint32_t r = 8u * j + (lane >> 2), q = lane & 3u;
+                const uint4 v = *reinterpret_cast<const uint4 *>(scratch + r * 80u + q * 16u);
+                const uint32_t prow = row - lane + r;
+                if (prow < p.m && cols_ok) {
+                    const size_t at = (size_t)prow * p.ld_out + f0 + q * 8u;
+#pragma unroll
+                    for (uint32_t k = 0; k + 1u < kMaxExchangeRanks; ++k) {
+                        if (k >= p.peers) break;
+                        *reinterpret_cast<uint4 *>(p.peer_out[k] + at) = v;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
 }
 
 // HALVES = 2: a CTA owns 256 rows (two 128-row accumulators over one dequantized weight tile).  HALVES = 1: 128
@@ -288,115 +343,12 @@ prefill_gemm_a4_kernel(const __grid_constant__ CUtensorMap x_map, const GemmPara
         // every tensor-core read of the operand stages has completed: their first bytes serve as 4 KB of scratch per warp
         uint8_t *scratch = stages + d * 4096u;
         const uint32_t row = m0 + half * 128u + sub * 32u + lane;  // this thread's row of the output
-        const bool row_ok = row < p.m;
 #pragma unroll 1
         for (uint32_t c = c_first; c < (stop == 0u ? c_first + c_count : 0u); ++c) {
             uint32_t acc[32];
             tmem_ld_32x32(tmem_base + ((sub * 32u) << 16) + half * kBN + c * 32u, acc);
             // columns of the accumulator are storage rows of the matrix: feature = 16 * tile + r
-            const uint32_t f0 = n_tile0 * 16u + c * 32u;
-            if (p.epilogue == kEpiSwiGlu) {
-                // storage tiles alternate up / gate (pair_halves): columns 0-15 up rows, 16-31 the gate rows
-                // of the same logical rows.  gated_act_mul.rs:80-95: silu in f32 -> bf16, product -> bf16
-                uint32_t packed[8];
-#pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    float o2[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float up = bf16_round(__uint_as_float(acc[i + e]));
-                        const float gate = bf16_round(__uint_as_float(acc[16 + i + e]));
-                        const float activated = bf16_round(gate / (1.0f + expf(-1.0f * gate)));
-                        o2[e] = up * activated;
-                    }
-                    packed[i >> 1] = f32x2_to_bf16x2(o2[0], o2[1]);
-                }
-                const uint32_t o0 = (f0 / 32u) * 16u;  // logical row of the pair
-                if (row_ok && o0 + 16u <= p.rows / 2u) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(p.out + (size_t)row * p.ld_out + o0);
-                    dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                }
-                if (p.peers && acc_ok) {
-                    // The same 32 x 16 block to the other ranks.  A lane holds 32 bytes of ITS row: stored from here, one
-                    // instruction would touch 32 rows with 16 bytes each, and over NVLink every such fragment is a packet
-                    // of its own.  Through the warp's scratch rows (48-byte pitch: conflict-free) the lanes regroup
-                    // so that two neighbours write one row's 32 contiguous bytes.
-                    uint4 *mine = reinterpret_cast<uint4 *>(scratch + lane * 48u);
-                    mine[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    mine[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                    __syncwarp();
-#pragma unroll
-                    for (uint32_t j = 0; j < 2u; ++j) {
-                        const uint32_t r = 16u * j + (lane >> 1), q = lane & 1u;
-                        const uint4 v = *reinterpret_cast<const uint4 *>(scratch + r * 48u + q * 16u);
-                        const uint32_t prow = row - lane + r;
-                        if (prow < p.m && o0 + 16u <= p.rows / 2u) {
-                            const size_t at = (size_t)prow * p.ld_out + o0 + q * 8u;
-#pragma unroll
-                            for (uint32_t k = 0; k + 1u < kMaxExchangeRanks; ++k) {
-                                if (k >= p.peers) break;
-                                *reinterpret_cast<uint4 *>(p.peer_out[k] + at) = v;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-            } else {
-                const bool cols_ok = f0 + 32u <= p.rows;
-                uint16_t *dst16 = p.out + (size_t)row * p.ld_out + f0;
-                uint32_t packed[16];
-                if (p.epilogue == kEpiResidual && row_ok && cols_ok) {
-                    const uint4 *src = reinterpret_cast<const uint4 *>(dst16);
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        const uint4 rv = src[q4];
-                        const uint32_t rr[4] = {rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int i = q4 * 8 + e * 2;
-                            const uint32_t y2 = f32x2_to_bf16x2(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]));
-                            packed[q4 * 4 + e] = f32x2_to_bf16x2(__uint_as_float(y2 << 16) + __uint_as_float(rr[e] << 16),
-                                                                 __uint_as_float(y2 & 0xffff0000u) +
-                                                                     __uint_as_float(rr[e] & 0xffff0000u));
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2)
-                        packed[i >> 1] = f32x2_to_bf16x2(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]));
-                }
-                if (row_ok && cols_ok) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(dst16);
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4)
-                        dst[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
-                }
-                if (p.peers && acc_ok) {
-                    // to the other ranks, regrouped through the warp's scratch rows (80-byte pitch) so that four
-                    // neighbouring lanes write one row's 64 contiguous bytes (see the gated branch)
-                    uint4 *mine = reinterpret_cast<uint4 *>(scratch + lane * 80u);
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4)
-                        mine[q4] = make_uint4(packed[4 * q4], packed[4 * q4 + 1], packed[4 * q4 + 2], packed[4 * q4 + 3]);
-                    __syncwarp();
-#pragma unroll
-                    for (uint32_t j = 0; j < 4u; ++j) {
-                        const uint32_t r = 8u * j + (lane >> 2), q = lane & 3u;
-                        const uint4 v = *reinterpret_cast<const uint4 *>(scratch + r * 80u + q * 16u);
-                        const uint32_t prow = row - lane + r;
-                        if (prow < p.m && cols_ok) {
-                            const size_t at = (size_t)prow * p.ld_out + f0 + q * 8u;
-#pragma unroll
-                            for (uint32_t k = 0; k + 1u < kMaxExchangeRanks; ++k) {
-                                if (k >= p.peers) break;
-                                *reinterpret_cast<uint4 *>(p.peer_out[k] + at) = v;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
+            store_block(p, row, n_tile0 * 16u + c * 32u, acc, scratch, lane, acc_ok);
         }
     }
     tc_fence_before();
@@ -405,6 +357,16 @@ prefill_gemm_a4_kernel(const __grid_constant__ CUtensorMap x_map, const GemmPara
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemColumns);
     }
+}
+
+// The contraction over weights that lie in memory as bf16 rows (pair_gemm.cuh).  Same values, same order of sums as the kernel above: the same bits.
+__global__ void __launch_bounds__(kPairThreads, 1)
+prefill_gemm_pair_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const GemmParams p) {
+    extern __shared__ uint8_t gemm_smem_raw[];
+    pair_gemm(x_map, w_map, p.groups, (p.m + kPairRows - 1u) / kPairRows, (p.row_tiles * 16u + kPairFeatures - 1u) / kPairFeatures,
+              p.error_word, gemm_smem_raw, [&](uint32_t row, uint32_t f0, const uint32_t (&acc)[32], uint8_t *scratch, uint32_t lane) {
+                  store_block(p, row, f0, acc, scratch, lane, true);
+              });
 }
 
 // ---------------------------------------------------------------------------------------- one or two row tiles
@@ -586,6 +548,26 @@ prefill_gemm_a4_thin_kernel(const __grid_constant__ CUtensorMap x_map, const Gem
 
 // ---------------------------------------------------------------------------------------- host side
 
+// Estimated us of the 256-feature tiles.  Over packed weights a step of 64 columns and wave of 256 rows takes 1.15, of 128 rows 0.75: the
+// dequantizing warps bound it.  Over unpacked ones a step of a round of pairs takes 0.4 (all SMs at the power limit), behind the
+// unpacking of 2.56 bytes a weight at 5 TB/s.  Measured, prompts of the 8b shape, packed and unpacked: 700 rows 17.1 and 17.4 ms, 1 000
+// rows 21.8 and 21.1, 3 000 rows 56.5 and 51.5; of the 0.6b shape 1 000 rows 4.70 and 4.22, 3 500 rows 12.3 and 9.8.
+struct WideTimes {
+    float packed, unpacked;
+};
+WideTimes wide_times(uint32_t features, uint32_t m, uint32_t groups) {
+    const uint32_t tiles = (features + kBN - 1u) / kBN, sms = 148u, tall = tiles * ((m + 255u) / 256u);
+    const float waves_256 = (float)((tall + sms - 1u) / sms), waves_128 = (float)((tiles * ((m + 127u) / 128u) + sms - 1u) / sms);
+    const float k = (float)groups, unpack = 2.5625f * 64.0f * k * (float)features / 5.0e6f, rounds = (float)((tall + sms / 2u - 1u) / (sms / 2u));
+    return {4.0f + k * std::min(1.15f * waves_256, 0.75f * waves_128), 8.0f + unpack + k * 0.4f * rounds};
+}
+// Setting gemm_unpack: 0 never, 1 by estimated times, 2 always.
+bool takes_unpacked(const WideTimes &t, uint32_t m) {
+    const uint32_t mode = tunables().gemm_unpack;
+    if (mode == 0u || m <= kPrefillSmallRows || tunables().gemm_stop_after) return false;
+    return mode == 2u || t.unpacked < t.packed;
+}
+
 // Setting gemm_thin: 0 never, 1 by estimated times, width + split that tile.  256-feature tiles take 1.15 us a step and wave of
 // 256 rows, 0.75 of 128 rows; measured, 77 rows: 1024 x 3072 39.6 -> 7.3 us, 4096 x 12288 136 -> 23, 6144 x 1024 gated 28.5 ->
 // 10; 301 rows: 41.4 -> 11.0, 141 -> 66, 29.2 -> 16; from about 600 rows the wide tiles fill the SMs and win.
@@ -593,13 +575,18 @@ ThinTile thin_tile(const GemmArgs &a) {
     const uint32_t mode = tunables().gemm_thin, groups = a.w->groups, features = a.whole_rows ? a.whole_rows : a.w->rows;
     if (mode == 0u || tunables().gemm_stop_after) return {};
     if (mode > 1u) return forced_thin_tile(mode, groups);
-    const uint32_t tiles = (features + kBN - 1u) / kBN, sms = 148u;
-    const uint32_t waves_256 = (tiles * ((a.m + 255u) / 256u) + sms - 1u) / sms, waves_128 = (tiles * ((a.m + 127u) / 128u) + sms - 1u) / sms;
-    const float wide = 4.0f + (float)groups * std::min(1.15f * (float)waves_256, 0.75f * (float)waves_128);
+    const WideTimes t = wide_times(features, a.m, groups);
+    const float wide = a.may_unpack && takes_unpacked(t, a.m) ? std::min(t.packed, t.unpacked) : t.packed;
     return pick_thin_tile(features, a.m, groups, wide, ThinSteps{{0.52f, 0.6f}, {0.6f, 0.85f}});
 }
 
 }  // namespace
+
+size_t prefill_gemm_unpacked_bytes(const GemmArgs &a) {
+    const QMatrix *w = a.w;
+    if (!w || w->format != kFmtAffine4 || thin_tile(a).width) return 0;
+    return takes_unpacked(wide_times(a.whole_rows ? a.whole_rows : w->rows, a.m, w->groups), a.m) ? (size_t)w->row_tiles * 16u * w->columns * 2u : 0u;
+}
 
 bool prefill_gemm_wide(const GemmArgs &a) { return !thin_tile(a).width; }
 
@@ -676,7 +663,17 @@ stark_b200_status prefill_gemm_launch(const GemmArgs &a, cudaStream_t stream) {
         return thin_launch(kernel, dim3((w->rows + thin.width - 1u) / thin.width, (a.m + 127u) / 128u, thin.split), kGemmThreads,
                            smem, stream, map, p);
     }
-    if (mode == 2u || (mode == 1u && cost_half < cost_full)) {
+    if (a.unpacked) {
+        CUtensorMap w_map;
+        const cuuint64_t w_dims[2] = {w->columns, w->row_tiles * 16u};
+        const cuuint32_t w_box[2] = {kBK, kPairFeatures / 2u};
+        if (encode(&w_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(a.unpacked), w_dims, strides, w_box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return STARK_B200_DEVICE_FAILURE;
+        static SmemOptIn once_pair;
+        if (stark_b200_status s = ensure_dynamic_smem(prefill_gemm_pair_kernel, (int)kPairSmem, once_pair)) return s;
+        if (stark_b200_status s = pair_launch(prefill_gemm_pair_kernel, w->row_tiles * 16u, a.m, sms, stream, map, w_map, p)) return s;
+    } else if (mode == 2u || (mode == 1u && cost_half < cost_full)) {
         static SmemOptIn once_half;
         if (stark_b200_status s = ensure_dynamic_smem(prefill_gemm_a4_kernel<1>, (int)kGemmSmem, once_half)) return s;
         prefill_gemm_a4_kernel<1><<<dim3(feature_tiles, (a.m + 127u) / 128u), kGemmThreads, kGemmSmem, stream>>>(map, p);

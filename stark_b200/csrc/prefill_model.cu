@@ -54,6 +54,37 @@ stark_b200_status ensure_chunk_buffers(Model *m) {
     return STARK_B200_OK;
 }
 
+// A layer's matrices in the order of their contractions.
+static void layer_matrices(const Model *m, const ModelLayer &L, const QMatrix *(&w)[4]) {
+    const bool tp = m->tp.size > 1u;
+    w[0] = L.qkv, w[1] = tp ? L.o_rows : L.o, w[2] = L.upgate, w[3] = tp ? L.down_rows : L.down;
+}
+
+// Where a pass of mrows rows writes a layer's matrices as bf16 rows: qkv and o, later [up; gate] and down, side by side in one buffer that
+// is kept for the passes to come (302 MB for the 8B shape); bytes[i] = 0 for those it reads packed.  The buffer is optional: with less
+// than a GiB to spare beside it (the sampler and the read-outs may still allocate) all stay packed.
+static void ensure_chunk_weights(Model *m, uint32_t mrows, size_t (&bytes)[4]) {
+    const QMatrix *w[4];
+    layer_matrices(m, m->layers[0], w);
+    for (int i = 0; i < 4; ++i) {
+        GemmArgs g{};
+        g.w = w[i];
+        g.m = mrows;
+        g.whole_rows = w[i]->rows * (m->tp.size > 1u ? m->tp.size : 1u);
+        g.may_unpack = true;
+        bytes[i] = prefill_gemm_unpacked_bytes(g);
+    }
+    const size_t need = std::max(bytes[0] + bytes[1], bytes[2] + bytes[3]);
+    size_t spare = 0, total = 0;
+    if (need > m->chunk_weights_bytes && cudaMemGetInfo(&spare, &total) == cudaSuccess &&
+        spare + m->chunk_weights_bytes >= need + ((size_t)1 << 30)) {
+        cudaFree(m->chunk_weights);  // waits for the launches that read it
+        m->chunk_weights_bytes = cudaMalloc(&m->chunk_weights, need) == cudaSuccess ? need : 0u;
+        if (!m->chunk_weights_bytes) m->chunk_weights = nullptr, cudaGetLastError();
+    }
+    if (need > m->chunk_weights_bytes) bytes[0] = bytes[1] = bytes[2] = bytes[3] = 0;
+}
+
 // Whether the batched path can take this model's prompt rows: one GPU, the recorded-launch token path, layer
 // matrices whose rows fill whole 128-feature tiles (examined once, at first use).
 bool model_batched_prefill_ready(Model *m) {
@@ -136,6 +167,8 @@ stark_b200_status model_rows_pass(Model *m, const uint32_t *tokens_device, uint3
         ++gathers;
         return tp_rows_gather_launch(m->tp_rows, ga, m->tp_rows_arrive, ctx->error_word, s);
     };
+    size_t unpacked_bytes[4];
+    ensure_chunk_weights(m, mrows, unpacked_bytes);
     if ((st = embed_rows_launch(m->embed, tokens_device, mrows, m->chunk_h, s)) != STARK_B200_OK) return st;
     for (uint32_t l = 0; l < c.layers; ++l) {
         auto &L = m->layers[l];
@@ -143,14 +176,23 @@ stark_b200_status model_rows_pass(Model *m, const uint32_t *tokens_device, uint3
         g.x_rows = kPrefillBatchRows;
         g.m = mrows;
         g.error_word = ctx->error_word;
+        g.may_unpack = true;
+        const QMatrix *w[4];
+        layer_matrices(m, L, w);
+        uint16_t *rows_of[4];  // their bf16 rows, nullptr: packed
+        for (int i = 0; i < 4; ++i)
+            rows_of[i] = unpacked_bytes[i] ? m->chunk_weights + (i & 1 ? unpacked_bytes[i - 1] / 2u : 0u) : nullptr;
         // qkv = W_qkv rmsnorm(h)
         if (fused_norm) {
             QmvMultiArgs q{L.qkv, m->chunk_h, c.hidden, mrows, m->chunk_qkv, qkv_n, L.attn_norm, c.eps, kEpiStore,
                            ctx->error_word, true};
             if ((st = qmv_multi_launch(q, s)) != STARK_B200_OK) return st;
         } else {
-            if ((st = rmsnorm_rows_launch(m->chunk_h, L.attn_norm, m->chunk_x, mrows, c.hidden, c.eps, s)) != STARK_B200_OK) return st;
-            g.w = L.qkv;
+            if ((st = rmsnorm_rows_unpack_launch(m->chunk_h, L.attn_norm, m->chunk_x, mrows, c.hidden, c.eps, {w[0], w[1]},
+                                                 {rows_of[0], rows_of[1]}, s)) != STARK_B200_OK)
+                return st;
+            g.w = w[0];
+            g.unpacked = rows_of[0];
             g.whole_rows = g.w->rows * ranks;
             g.x = m->chunk_x;
             g.out = m->chunk_qkv;
@@ -172,7 +214,8 @@ stark_b200_status model_rows_pass(Model *m, const uint32_t *tokens_device, uint3
                                true)) != STARK_B200_OK)
             return st;
         // h = bf16(bf16(W_o attn) + h); tensor parallel: this rank's columns of h, in place, then gathered
-        g.w = tp ? L.o_rows : L.o;
+        g.w = w[1];
+        g.unpacked = rows_of[1];
         g.whole_rows = g.w->rows * ranks;
         g.x = attn_rows;
         g.out = m->chunk_h + (size_t)rank * h_slice;
@@ -193,8 +236,11 @@ stark_b200_status model_rows_pass(Model *m, const uint32_t *tokens_device, uint3
                            ctx->error_word, true};
             if ((st = qmv_multi_launch(q, s)) != STARK_B200_OK) return st;
         } else {
-            if ((st = rmsnorm_rows_launch(m->chunk_h, L.mlp_norm, m->chunk_x, mrows, c.hidden, c.eps, s)) != STARK_B200_OK) return st;
-            g.w = L.upgate;
+            if ((st = rmsnorm_rows_unpack_launch(m->chunk_h, L.mlp_norm, m->chunk_x, mrows, c.hidden, c.eps, {w[2], w[3]},
+                                                 {rows_of[2], rows_of[3]}, s)) != STARK_B200_OK)
+                return st;
+            g.w = w[2];
+            g.unpacked = rows_of[2];
             g.whole_rows = g.w->rows * ranks;
             g.x = m->chunk_x;
             g.out = act_slice;
@@ -209,7 +255,8 @@ stark_b200_status model_rows_pass(Model *m, const uint32_t *tokens_device, uint3
                                pushed ? 0u : c.inter, false)) != STARK_B200_OK)
             return st;
         // h = bf16(bf16(W_down act) + h)
-        g.w = tp ? L.down_rows : L.down;
+        g.w = w[3];
+        g.unpacked = rows_of[3];
         g.whole_rows = g.w->rows * ranks;
         g.x = m->chunk_act;
         g.out = m->chunk_h + (size_t)rank * h_slice;

@@ -3,6 +3,7 @@
 // formulas, same rounding points -- so that a prompt row costs the same arithmetic whichever path takes it.
 #include <algorithm>
 
+#include "a4_record.cuh"
 #include "device_math.cuh"
 #include "prefill.cuh"
 #include "tunables.cuh"
@@ -70,13 +71,11 @@ __global__ void embed_rows_kernel(const uint8_t *__restrict__ data, uint32_t row
 // bf16(x * rms_inv) * bf16(weight) rounded to bf16.  One CTA per row, the row held in registers.
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxChunks = 6;  // 8 elements each: rows of up to 12288
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const uint16_t *h,
-                                                                    const float *__restrict__ weight,
-                                                                    uint16_t *out, uint32_t d, float eps,
-                                                                    uint32_t in_stride, uint32_t out_stride) {
+__device__ __forceinline__ void rmsnorm_row(uint32_t row, const uint16_t *h, const float *__restrict__ weight, uint16_t *out, uint32_t d,
+                                            float eps, uint32_t in_stride, uint32_t out_stride) {
     __shared__ float red[kNormThreads / 32];
     const uint32_t tid = threadIdx.x, chunks = d / 8u;
-    const uint4 *src = reinterpret_cast<const uint4 *>(h + (size_t)blockIdx.x * in_stride);
+    const uint4 *src = reinterpret_cast<const uint4 *>(h + (size_t)row * in_stride);
     pdl_launch_dependents();
     pdl_wait();  // the rows come from the launch before this one
     uint4 v[kNormMaxChunks];
@@ -100,7 +99,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const uint16
 #pragma unroll
     for (int i = 0; i < kNormThreads / 32; ++i) total += red[i];
     const float rms_inv = 1.0f / sqrtf(total / (float)d + eps);
-    uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)blockIdx.x * out_stride);
+    uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)row * out_stride);
 #pragma unroll
     for (int r = 0; r < kNormMaxChunks; ++r) {
         const uint32_t c = tid + r * kNormThreads;
@@ -118,6 +117,26 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const uint16
         }
         dst[c] = make_uint4(o[0], o[1], o[2], o[3]);
     }
+}
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const uint16_t *h, const float *__restrict__ weight, uint16_t *out,
+                                                                    uint32_t d, float eps, uint32_t in_stride, uint32_t out_stride) {
+    rmsnorm_row(blockIdx.x, h, weight, out, d, eps, in_stride, out_stride);
+}
+// The first `unpackers` CTAs write matrices as bf16 rows, the others a row each.
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_unpack_kernel(const uint16_t *h, const float *__restrict__ weight,
+                                                                           uint16_t *out, uint32_t d, float eps, const UnpackJobs jobs,
+                                                                           uint32_t unpackers) {
+    if (blockIdx.x >= unpackers) {
+        rmsnorm_row(blockIdx.x - unpackers, h, weight, out, d, eps, d, d);
+        return;
+    }
+    pdl_launch_dependents();
+    pdl_wait();  // the launch before this one may still read the rows that are written here
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        if (jobs.out[i])
+            unpack_records(jobs.w[i], jobs.out[i], jobs.row_tiles[i], jobs.groups[i], blockIdx.x * (kNormThreads / 32u) + (threadIdx.x >> 5),
+                           unpackers * (kNormThreads / 32u));
 }
 
 // ------------------------------------------------------------------------------------------ row arg-max
@@ -680,6 +699,24 @@ stark_b200_status rmsnorm_rows_launch(const uint16_t *h, const float *weight, ui
         return STARK_B200_INVALID_ARGUMENT;
     SB_CUDA(launch_dependent(rmsnorm_rows_kernel, dim3(m), dim3(kNormThreads), 0, stream, h, weight, out, d, eps,
                              in_stride ? in_stride : d, out_stride ? out_stride : d));
+    return STARK_B200_OK;
+}
+
+stark_b200_status rmsnorm_rows_unpack_launch(const uint16_t *h, const float *weight, uint16_t *out, uint32_t m, uint32_t d, float eps,
+                                             const QMatrix *const (&w)[2], uint16_t *const (&to)[2], cudaStream_t stream) {
+    if (!to[0] && !to[1]) return rmsnorm_rows_launch(h, weight, out, m, d, eps, stream);
+    if (!h || !weight || !out || m == 0 || d % 8u != 0 || d > (uint32_t)kNormThreads * kNormMaxChunks * 8u) return STARK_B200_INVALID_ARGUMENT;
+    UnpackJobs jobs{};
+    uint32_t records = 0;
+    for (int i = 0; i < 2; ++i) {
+        if (!to[i]) continue;
+        if (w[i]->format != kFmtAffine4) return STARK_B200_UNSUPPORTED;
+        jobs.w[i] = w[i]->data, jobs.out[i] = to[i], jobs.row_tiles[i] = w[i]->row_tiles, jobs.groups[i] = w[i]->groups;
+        records = std::max(records, w[i]->row_tiles * w[i]->groups);
+    }
+    const uint32_t unpackers = std::min((records + 15u) / 16u, 148u * 6u);
+    SB_CUDA(launch_dependent(rmsnorm_rows_unpack_kernel, dim3(unpackers + m), dim3(kNormThreads), 0, stream, h, weight, out, d, eps, jobs,
+                             unpackers));
     return STARK_B200_OK;
 }
 

@@ -270,3 +270,29 @@ def test_several_rows_matvec_swiglu():
     assert got.shape == (m, inter)
     assert (got != own).mean() < 0.01 and _rel(got, own).max() < REL_TOL
     assert ops.take_device_error() == 0
+
+
+@pytest.mark.parametrize("rows", [17, 256, 257, 700])
+@pytest.mark.parametrize("hidden,q_heads,inter", [(384, 3, 640), (256, 2, 128)])
+def test_unpacked_weights_leave_the_same_bits(rows, hidden, q_heads, inter):
+    """The contraction over weights unpacked to bf16 rows, on pairs of SMs, against the one that dequantizes its own tiles: the same
+    values added in the same order.  Features and rows past the last whole tile, fewer steps than stages, more tiles than a pair
+    has accumulators."""
+    from stark_b200.engine import DenseModel
+    from stark_b200.ops import take_device_error
+    cfg = dict(layers=2, hidden=hidden, q_heads=q_heads, kv_heads=1, head_dim=128, inter=inter, vocab=1024, tied=False, eps=1e-6, rope_theta=1e6)
+    model = DenseModel.load(cfg, S.dense_weights(cfg, seed=2, zero_point=7.5), context_tokens=rows + 32)
+    prompt = S.prompt(cfg, rows + 1, seed=3)
+    got = []
+    try:
+        _set("gemm_thin", 0)
+        for unpack in (0, 2):
+            _set("gemm_unpack", unpack)
+            model.reset()
+            model.prefill(prompt)
+            got.append(model.logits_bf16().copy())
+    finally:
+        _set("gemm_thin", 1)
+        _set("gemm_unpack", 1)
+    assert take_device_error() == 0
+    assert np.array_equal(got[0], got[1])
