@@ -818,6 +818,7 @@ stark_b200_status qmv_launch(const QmvArgs &a, cudaStream_t stream) {
         return STARK_B200_UNSUPPORTED;
     if (m->columns > kMaxColumns) return STARK_B200_UNSUPPORTED;
     if (qmv_short_takes(a)) return qmv_short_launch(a, stream);
+    if (qmv_slice_takes(a)) return qmv_slice_launch(a, stream);
 
     const bool split = a.io_type == STARK_B200_F32;
     const Tunables &tune = tunables();

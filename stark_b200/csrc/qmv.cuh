@@ -120,6 +120,13 @@ stark_b200_status qmv_launch(const QmvArgs &args, cudaStream_t stream);
 // The form for matrices that are requested whole (qmv_short.cu); qmv_launch takes it where it fits.
 bool qmv_short_takes(const QmvArgs &args);
 stark_b200_status qmv_short_launch(const QmvArgs &args, cudaStream_t stream);
+// The form whose warps own a slice of the columns each (qmv_slice.cu), for one row and for a handful; qmv_launch and qmv_multi_launch
+// take it where it fits.
+bool qmv_slice_takes(const QmvArgs &args);
+stark_b200_status qmv_slice_launch(const QmvArgs &args, cudaStream_t stream);
+struct QmvMultiArgs;
+bool qmv_slice_multi_takes(const QmvMultiArgs &args);
+stark_b200_status qmv_slice_multi_launch(const QmvMultiArgs &args, cudaStream_t stream);
 // Ring-stage geometry for a matrix with `groups` column groups: records per stage, records per
 // consumer warp, and whether the stage is ragged (needs per-record predicates).
 void qmv_pick_stage(uint32_t groups, uint32_t *records, uint32_t *rpw, bool *pred);

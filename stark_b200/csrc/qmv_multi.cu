@@ -408,6 +408,7 @@ stark_b200_status qmv_multi_launch(const QmvMultiArgs &a, cudaStream_t stream) {
     if (a.epilogue != kEpiStore && a.epilogue != kEpiResidual && a.epilogue != kEpiSwiGlu) return STARK_B200_UNSUPPORTED;
     if ((a.epilogue == kEpiSwiGlu) != (w->pair_halves != 0)) return STARK_B200_INVALID_ARGUMENT;
     if ((reinterpret_cast<uintptr_t>(a.x) & 15u) || (a.x_stride % 8u) != 0) return STARK_B200_INVALID_ARGUMENT;
+    if (qmv_slice_multi_takes(a)) return qmv_slice_multi_launch(a, stream);
     MultiParams p{};
     uint32_t smem = 0;
     multi_geometry(w, a.m, &p, &smem);

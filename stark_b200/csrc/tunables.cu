@@ -20,6 +20,7 @@ const Entry kEntries[] = {
     {"qmv_ctas_per_sm", "STARK_B200_QMV_CTAS", &Tunables::qmv_ctas_per_sm, 0u, 0u, 2u},
     {"qmv_fold", "STARK_B200_QMV_FOLD", &Tunables::qmv_fold, 0u, 0u, 2u},
     {"qmv_short", "STARK_B200_QMV_SHORT", &Tunables::qmv_short, 1u, 0u, 1u},
+    {"qmv_slice", "STARK_B200_QMV_SLICE", &Tunables::qmv_slice, 1u, 0u, 1u},
     {"attn_bufs", "STARK_B200_ATTN_BUFS", &Tunables::attn_bufs, 3u, 2u, 3u},
     {"attn_splits", "STARK_B200_ATTN_SPLITS", &Tunables::attn_splits, 0u, 0u, 32u},
     {"attn_regs", "STARK_B200_ATTN_REGS", &Tunables::attn_regs, 96u, 96u, 128u},

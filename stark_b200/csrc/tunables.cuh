@@ -13,6 +13,7 @@ struct Tunables {
     uint32_t qmv_ctas_per_sm;     // STARK_B200_QMV_CTAS    0 = the shape's own count
     uint32_t qmv_short;           // STARK_B200_QMV_SHORT   1: matrices that fit the SMs whole are requested whole (qmv_short.cu), 0: streamed
     uint32_t qmv_fold;            // STARK_B200_QMV_FOLD    0 | 1 | 2
+    uint32_t qmv_slice;           // STARK_B200_QMV_SLICE   1: warps own slices of the columns (qmv_slice.cu) where they divide them, 0: shared ring
     uint32_t attn_bufs;           // STARK_B200_ATTN_BUFS   2 | 3
     uint32_t attn_splits;         // STARK_B200_ATTN_SPLITS 0 = chosen from the head count
     uint32_t attn_regs;           // STARK_B200_ATTN_REGS   96 | 128 registers per attention thread

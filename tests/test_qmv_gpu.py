@@ -162,3 +162,47 @@ def test_invalid_arguments_are_rejected():
         q.matvec(np.zeros(63, np.uint16))
     with pytest.raises(StarkB200Error):
         QMatrix.from_affine(w["codes"], w["scales"], w["biases"], 16, 64, group=32)
+
+
+@pytest.mark.parametrize("rows,columns", [(16, 1024), (1000, 2048), (4800, 3072), (6144, 4096), (100, 8192), (2048, 12288), (9488, 5120)])
+def test_column_slices(rows, columns):
+    """Warps that own slices of the columns (two to eight groups of 64, one to three chunks), against the shared ring: one row plain and
+    gated, two to eight rows with and without the norm.  A last row tile in part, fewer tiles than CTAs, more than a round of them.  The
+    same products up to an offset the group sums take out again, f32 sums formed in another order, one rounding to bf16; and no further
+    from the 64-bit result."""
+    from stark_b200 import _lib
+    from stark_b200.ops import QMatrix, qmv_swiglu, take_device_error
+    w = S.matvec_case(seed=9 + rows, rows=rows, columns=columns)
+    make = lambda pair: QMatrix.from_affine(w["codes"], w["scales"], w["biases"], rows, columns, pair_halves=pair)  # noqa: E731
+    plain, pair = make(False), make(True) if rows % 32 == 0 else None
+    rng = np.random.default_rng(rows)
+    several = {m: S.bf16_normal(rng, m * columns).reshape(m, columns) for m in (2, 5, 8)}
+    weight = (1.0 + 0.1 * rng.standard_normal(columns)).astype(np.float32)
+    seen = []
+    try:
+        _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", 0), "set_tunable")
+        for sliced in (0, 1):
+            _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_slice", sliced), "set_tunable")
+            out = [plain.matvec(w["x"]), qmv_swiglu(pair, w["x"]) if pair else None]
+            for m, x in several.items():
+                out.append(plain.matvec_rows(x))
+                if columns <= 4096:
+                    out.append(plain.matvec_rows(x, norm_weight=weight))
+                    out.append(plain.matvec_rows(x, epilogue=1, residual=S.bf16_normal(np.random.default_rng(m), m * rows).reshape(m, rows)))
+                    if pair:
+                        out.append(pair.matvec_rows(x, epilogue=2, norm_weight=weight))
+            seen.append(out)
+    finally:
+        _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_short", 1), "set_tunable")
+        _lib.check(_lib.load().stark_b200_set_tunable(b"qmv_slice", 1), "set_tunable")
+    assert take_device_error() == 0
+    for ring, sliced in zip(*seen):
+        if ring is None:
+            continue
+        assert (ring != sliced).mean() < 0.02
+        assert _rel_err(sliced, ring).max() <= 3 * 2.0 ** -7  # a unit of the last place; of both factors and their product
+    codes = O.unpack_codes(w["codes"], 4, rows * columns).reshape(rows, columns // 64, 64).astype(np.float64)
+    scale, bias = (O.bf16_to_f32(w[k]).astype(np.float64).reshape(rows, -1, 1) for k in ("scales", "biases"))
+    exact = (codes * scale + bias).reshape(rows, columns) @ O.bf16_to_f32(w["x"]).astype(np.float64)
+    off = [np.linalg.norm(O.bf16_to_f32(out[0]).astype(np.float64) - exact) for out in seen]
+    assert off[1] <= 1.02 * off[0]   # rounding to bf16 is the error: the few results that round the other way move it this much
