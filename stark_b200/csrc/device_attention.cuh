@@ -30,7 +30,11 @@ struct AttnShared {
     uint16_t (*q_s)[kHeadDim];        // [kMaxGqa] q after norm + RoPE, bf16
     uint16_t *knew, *vnew;            // [kHeadDim] the appended key / value row
     float (*ml_s)[kMaxGqa][2];        // [kAttnWarps] per-warp (max, sum)
+    float *recv;                      // cluster form: [splits][this CTA's share of the outputs], every split's part of them
+    float2 *stats;                    // and [splits][heads of the group] (max, sum)
 };
+// Of the cluster form, behind the rest: the parts and the statistics of up to 16 splits.
+__host__ __device__ constexpr uint32_t attn_cluster_bytes(uint32_t gqa) { return (gqa * kHeadDim + 16u) * 4u + 16u * gqa * 8u; }
 // nbuf = K / V tile pairs in flight (2: double buffered; 3: a split of up to three pages is fetched whole
 // before the new row exists).
 __host__ __device__ constexpr uint32_t attn_shared_bytes(uint32_t nbuf) {
@@ -46,6 +50,8 @@ __device__ inline AttnShared carve_attn_shared(uint8_t *base /* 128-byte aligned
     s.knew = reinterpret_cast<uint16_t *>(base + tile_bytes + kMaxGqa * kHeadDim * 2u);
     s.vnew = s.knew + kHeadDim;
     s.ml_s = reinterpret_cast<float(*)[kMaxGqa][2]>(s.vnew + kHeadDim);
+    s.recv = reinterpret_cast<float *>(s.ml_s + kAttnWarps);
+    s.stats = nullptr;
     return s;
 }
 
@@ -53,12 +59,13 @@ __device__ inline AttnShared carve_attn_shared(uint8_t *base /* 128-byte aligned
 // and the per-lane constants of the head norm and RoPE at the row's position.
 struct AttnPrefetch {
     uint32_t pos;
+    int32_t page;  // of the split's tile `lane`
     HeadConsts cq, ck;
 };
 
-__device__ inline void attn_issue_tile(const AttnParams &p, uint32_t h, uint32_t block, uint32_t buf, uint8_t *tiles,
+__device__ inline void attn_issue_tile(const AttnParams &p, uint32_t h, int32_t block_page, uint32_t buf, uint8_t *tiles,
                                        uint32_t tid) {
-    const size_t page = ((size_t)p.block_table[block] * p.kv_heads + h) * kPageTokens * kHeadDim;
+    const size_t page = ((size_t)block_page * p.kv_heads + h) * kPageTokens * kHeadDim;
     const uint8_t *ksrc = reinterpret_cast<const uint8_t *>(p.keys + page);
     const uint8_t *vsrc = reinterpret_cast<const uint8_t *>(p.values + page);
     uint8_t *kd = tiles + (size_t)(buf * 2u) * kTileBytes, *vd = kd + kTileBytes;
@@ -86,9 +93,12 @@ __device__ inline void attention_prefetch(const AttnParams &p, uint32_t split, u
     uint32_t b0, b1;
     attn_split_range(p, split, pos, b0, b1);
     if (tid < (uint32_t)kAttnThreads) {
+        // the pages of the split's first 32 tiles, a lane each: no tile waits for its entry of the table
+        pf.page = b0 + (tid & 31u) < b1 ? p.block_table[b0 + (tid & 31u)] : 0;
 #pragma unroll
         for (uint32_t i = 0; i < (uint32_t)NBUF; ++i) {
-            if (b1 > b0 + i) attn_issue_tile(p, h, b0 + i, i, sm.tiles, tid);
+            const int32_t page = __shfl_sync(0xffffffffu, pf.page, i);
+            if (b1 > b0 + i) attn_issue_tile(p, h, page, i, sm.tiles, tid);
             cp_async_commit();
         }
         const float *cosr = p.rope_cos ? p.rope_cos + (size_t)pos * kHeadDim : nullptr;
@@ -96,6 +106,30 @@ __device__ inline void attention_prefetch(const AttnParams &p, uint32_t split, u
         pf.cq = load_head_consts(p.q_norm, cosr, sinr, tid & 31u);
         pf.ck = load_head_consts(p.k_norm, cosr, sinr, tid & 31u);
     }
+}
+
+// The rows a thread's warp norms and rotates -- the query heads of the group, then the new key row -- and its part of the new value
+// row.  All of them are requested before the first is used, and by the kernel before it looks at the position again.
+constexpr uint32_t kMaxHeadsPerWarp = (kMaxGqa + 1u + kAttnWarps - 1u) / kAttnWarps;
+static_assert(kMaxHeadsPerWarp == 3u, "attention_partial picks among three");
+struct AttnRows {
+    uint32_t lo[kMaxHeadsPerWarp], hi[kMaxHeadsPerWarp];
+    uint2 v;
+};
+__device__ inline AttnRows attention_rows(const AttnParams &p, uint32_t h, uint32_t tid) {
+    const uint32_t lane = tid & 31u, warp = tid >> 5, G = p.gqa;
+    AttnRows r;
+    r.v = make_uint2(0u, 0u);
+#pragma unroll
+    for (uint32_t i = 0; i < kMaxHeadsPerWarp; ++i) {
+        const uint32_t hh = warp + i * kAttnWarps;
+        r.lo[i] = r.hi[i] = 0u;
+        if (tid >= (uint32_t)kAttnThreads || hh > G) continue;
+        load_head_row(p.qkv + (size_t)(hh < G ? h * G + hh : p.q_heads + h) * kHeadDim, lane, r.lo[i], r.hi[i]);
+        if (hh == G)
+            r.v = __ldcg(reinterpret_cast<const uint2 *>(p.qkv + (size_t)(p.q_heads + p.kv_heads + h) * kHeadDim + 4u * lane));
+    }
+    return r;
 }
 
 // Split `split` of KV head `h`: writes the partial (o, max, sum) of the G query heads of the group to
@@ -107,9 +141,11 @@ __device__ inline void attention_prefetch(const AttnParams &p, uint32_t split, u
 // are the M rows) and the same online softmax in f32, then O += P V for its own 32 of the 128 output
 // dims, with P carried as bf16 hi + lo so that the weights keep ~16 bits.  Warps only synchronise to
 // hand tile buffers over.  Inputs written by other CTAs of a running kernel are read with ld.cg.
-template <int BAR_ID, int BAR_THREADS, int NBUF = 2>
+// CLUSTER: the splits of a head are the CTAs of a cluster.  Every CTA owns an equal share of the group's outputs; instead of a partial
+// in memory, a split leaves its part of every share, and its statistics, in the owners' shared memory (attention_cluster_merge).
+template <int BAR_ID, int BAR_THREADS, int NBUF = 2, bool CLUSTER = false>
 __device__ inline void attention_partial(const AttnParams &p, uint32_t split, uint32_t h, uint32_t pos,
-                                         const AttnShared &sm, uint32_t tid, const AttnPrefetch &pf) {
+                                         const AttnShared &sm, uint32_t tid, const AttnPrefetch &pf, const AttnRows &rows) {
     const uint32_t lane = tid & 31u, warp = tid >> 5, G = p.gqa;
     const uint32_t g = lane >> 2, t = lane & 3u;
     const bool worker = tid < (uint32_t)kAttnThreads;
@@ -122,35 +158,17 @@ __device__ inline void attention_partial(const AttnParams &p, uint32_t split, ui
     uint8_t *tiles = sm.tiles;
 
     // Norm + RoPE: one warp per head (the G query heads, then the new key row on the owner split).
-    // All rows a warp needs are requested before the first is used: the owner split's extra row must not
-    // cost a second trip to memory, because the slowest CTA sets the kernel's duration.
     if (worker) {
-        constexpr uint32_t kMaxHeadsPerWarp = (kMaxGqa + 1u + kAttnWarps - 1u) / kAttnWarps;
-        uint32_t raw_lo[kMaxHeadsPerWarp], raw_hi[kMaxHeadsPerWarp];
-        uint2 vv = make_uint2(0u, 0u);
-#pragma unroll
+#pragma unroll 1  // one copy of the code: a launch fetches all of it anew
         for (uint32_t i = 0; i < kMaxHeadsPerWarp; ++i) {
             const uint32_t hh = warp + i * kAttnWarps;
-            const uint16_t *row = nullptr;
-            if (hh < G) row = p.qkv + (size_t)(h * G + hh) * kHeadDim;
-            else if (hh == G && owner) row = p.qkv + (size_t)(p.q_heads + h) * kHeadDim;
-            raw_lo[i] = raw_hi[i] = 0u;
-            if (row) load_head_row(row, lane, raw_lo[i], raw_hi[i]);
-            if (hh == G && owner)
-                vv = __ldcg(reinterpret_cast<const uint2 *>(p.qkv + (size_t)(p.q_heads + p.kv_heads + h) * kHeadDim +
-                                                            4u * lane));
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < kMaxHeadsPerWarp; ++i) {
-            const uint32_t hh = warp + i * kAttnWarps;
-            if (hh < G) {
-                head_norm_rope_regs(raw_lo[i], raw_hi[i], pf.cq, p.q_norm != nullptr, p.rope_cos != nullptr, p.eps, lane,
-                                    sm.q_s[hh]);
-            } else if (hh == G && owner) {
-                head_norm_rope_regs(raw_lo[i], raw_hi[i], pf.ck, p.k_norm != nullptr, p.rope_cos != nullptr, p.eps, lane,
-                                    sm.knew);
-                *reinterpret_cast<uint2 *>(sm.vnew + 4u * lane) = vv;
-            }
+            if (hh > G || (hh == G && !owner)) break;
+            const bool key = hh == G;
+            HeadConsts c = pf.cq;
+            if (key) c = pf.ck;
+            const uint32_t lo = i == 0 ? rows.lo[0] : (i == 1 ? rows.lo[1] : rows.lo[2]), hi = i == 0 ? rows.hi[0] : (i == 1 ? rows.hi[1] : rows.hi[2]);
+            head_norm_rope_regs(lo, hi, c, (key ? p.k_norm : p.q_norm) != nullptr, p.rope_cos != nullptr, p.eps, lane, key ? sm.knew : sm.q_s[hh]);
+            if (key) *reinterpret_cast<uint2 *>(sm.vnew + 4u * lane) = rows.v;
         }
     }
     named_bar_sync(BAR_ID, BAR_THREADS);
@@ -211,14 +229,16 @@ __device__ inline void attention_partial(const AttnParams &p, uint32_t split, ui
         }
         const uint32_t valid = min(kPageTokens, seq_len - blk * kPageTokens);
         if (worker && k0 < valid) {  // a slab with no key in range would have no finite maximum
-            float sc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            float sc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sd[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // two chains: even and odd kk
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 // matrices: (keys 0-7, dims 0-7), (keys 8-15, dims 0-7), (keys 0-7, dims 8-15), (keys 8-15, dims 8-15)
                 uint32_t ka[4];
                 ldmatrix_x4(ka, kt + (k0 + (lmat & 1u) * 8u + lrow) * kTileRowBytes + (kk * 16u + (lmat >> 1) * 8u) * 2u);
-                mma_m16n8k16_bf16(sc, ka[0], ka[1], ka[2], ka[3], qb[kk][0], qb[kk][1]);
+                mma_m16n8k16_bf16(kk & 1 ? sd : sc, ka[0], ka[1], ka[2], ka[3], qb[kk][0], qb[kk][1]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sc[i] += sd[i];
             // sc[0], sc[1]: key k0+g, heads 2t, 2t+1;  sc[2], sc[3]: key k0+g+8
             const bool va = k0 + g < valid, vb = k0 + g + 8u < valid;
             float e[4], factor[2];
@@ -233,11 +253,7 @@ __device__ inline void attention_partial(const AttnParams &p, uint32_t split, ui
                 factor[j] = m_run[j] == -INFINITY ? 0.0f : expf(m_run[j] - m_new);
                 e[j] = expf(sa - m_new);
                 e[2 + j] = expf(sb2 - m_new);
-                float ts = e[j] + e[2 + j];
-                ts += __shfl_xor_sync(0xffffffffu, ts, 4);
-                ts += __shfl_xor_sync(0xffffffffu, ts, 8);
-                ts += __shfl_xor_sync(0xffffffffu, ts, 16);
-                l_run[j] = l_run[j] * factor[j] + ts;
+                l_run[j] = l_run[j] * factor[j] + (e[j] + e[2 + j]);  // this lane's keys; the lanes are added up at the end
                 m_run[j] = m_new;
             }
 #pragma unroll
@@ -269,12 +285,18 @@ __device__ inline void attention_partial(const AttnParams &p, uint32_t split, ui
         }
         named_bar_sync(BAR_ID, BAR_THREADS);  // the buffer of this tile is free for tile + NBUF
         if (worker) {
-            if (tile + (uint32_t)NBUF < ntiles) attn_issue_tile(p, h, b0 + tile + (uint32_t)NBUF, buf, tiles, tid);
+            const uint32_t next = tile + (uint32_t)NBUF;
+            const int32_t page = next < 32u ? __shfl_sync(0xffffffffu, pf.page, next) : (next < ntiles ? p.block_table[b0 + next] : 0);
+            if (next < ntiles) attn_issue_tile(p, h, page, buf, tiles, tid);
             cp_async_commit();
         }
     }
 
     // ---- merge the four warps' states, publish this split's partial (o, max, sum) ----
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int o = 4; o < 32; o *= 2) l_run[j] += __shfl_xor_sync(0xffffffffu, l_run[j], o);
     if (worker && g == 0) {
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -305,6 +327,36 @@ __device__ inline void attention_partial(const AttnParams &p, uint32_t split, ui
         }
     }
     named_bar_sync(BAR_ID, BAR_THREADS);
+    if constexpr (CLUSTER) {
+        const uint32_t share = (G * kHeadDim + p.splits - 1u) / p.splits;
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // arrived for at its start: every CTA of the cluster runs
+        const auto at = [](const void *local, uint32_t cta) {
+            uint32_t a;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(cta));
+            return a;
+        };
+        for (uint32_t i = tid; i < G * kHeadDim; i += kAttnThreads) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) acc += o_s[(size_t)w * G * kHeadDim + i];
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at(sm.recv + split * share + i % share, i / share)), "f"(acc) : "memory");
+        }
+        for (uint32_t i = tid; i < G * p.splits; i += kAttnThreads) {
+            const uint32_t head = i / p.splits;
+            float mx = -INFINITY, l = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) mx = fmaxf(mx, sm.ml_s[w][head][0]);
+#pragma unroll
+            for (int w = 0; w < kAttnWarps; ++w) {
+                const float mw = sm.ml_s[w][head][0];
+                l += mw == -INFINITY ? 0.0f : sm.ml_s[w][head][1] * expf(mw - mx);
+            }
+            asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(at(sm.stats + split * G + head, i % p.splits)), "f"(mx), "f"(l)
+                         : "memory");
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return;
+    }
     const uint32_t stride = kHeadDim + 2u;
     float *mine = p.scratch + ((size_t)(h * p.splits + split) * G) * stride;
     if (worker) {
@@ -330,6 +382,30 @@ __device__ inline void attention_partial(const AttnParams &p, uint32_t split, ui
         __threadfence();
     }
     named_bar_sync(BAR_ID, BAR_THREADS);
+}
+
+// This CTA's share of the outputs of KV head `h` from what the cluster's splits left here: a few lanes an output, each some splits.
+__device__ inline void attention_cluster_merge(const AttnParams &p, uint32_t split, uint32_t h, const AttnShared &sm, uint32_t tid) {
+    const uint32_t G = p.gqa, share = (G * kHeadDim + p.splits - 1u) / p.splits, all = G * kHeadDim;
+    uint32_t lanes = 1;
+    while (2u * lanes * share <= (uint32_t)kAttnThreads && lanes < 16u) lanes *= 2u;
+    const uint32_t out = min(tid / lanes, share - 1u), head = min(split * share + out, all - 1u) / kHeadDim;
+    float mx = -INFINITY;
+    for (uint32_t s = tid % lanes; s < p.splits; s += lanes) mx = fmaxf(mx, sm.stats[s * G + head].x);
+    for (uint32_t o = 1; o < lanes; o *= 2u) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float acc = 0.0f, l = 0.0f;
+    for (uint32_t s = tid % lanes; s < p.splits; s += lanes) {
+        const float2 st = sm.stats[s * G + head];
+        const float w = st.x == -INFINITY ? 0.0f : expf(st.x - mx);
+        acc = fmaf(w, sm.recv[s * share + out], acc);
+        l = fmaf(w, st.y, l);
+    }
+    for (uint32_t o = 1; o < lanes; o *= 2u) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+    }
+    if (tid % lanes == 0 && tid / lanes < share && split * share + out < all)
+        p.out[(size_t)h * G * kHeadDim + split * share + out] = f32_to_bf16_bits(acc * (1.0f / l));
 }
 
 // Merges the `splits` partials of KV head `h` into p.out: one warp per query head, lane s holding the

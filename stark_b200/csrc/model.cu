@@ -97,6 +97,7 @@ stark_b200_status model_create(const stark_b200_dense_config &c, Model **out) {
     // splits than that start cold.
     m->attn_splits = default_attn_splits(c.kv_heads);
     if (tunables().attn_splits) m->attn_splits = tunables().attn_splits;  // tuning: CTAs per KV head
+    else m->attn_cluster = attention_cluster_ctas(c.q_heads, c.kv_heads);
     if ((st = dmalloc(&m->h, c.hidden)) != STARK_B200_OK) return fail(st);
     if ((st = dmalloc(&m->h_alt, c.hidden)) != STARK_B200_OK) return fail(st);
     if ((st = dmalloc(&m->qkv, qkv_n)) != STARK_B200_OK) return fail(st);
@@ -294,6 +295,7 @@ static stark_b200_status issue_token(Model *m, bool full, uint32_t *launches) {
         at.q_heads = c.q_heads;
         at.kv_heads = c.kv_heads;
         at.splits = m->attn_splits;
+        at.cluster = m->attn_cluster;
         at.scratch = m->attn_scratch;
         at.counters = m->attn_counters;
         at.error_word = ctx->error_word;
@@ -660,6 +662,7 @@ static stark_b200_status dense_launch_persistent(Model *m, bool full) {
 
 static void dense_retune(Model *m) {
     m->attn_splits = tunables().attn_splits ? tunables().attn_splits : default_attn_splits(m->cfg.kv_heads);
+    m->attn_cluster = tunables().attn_splits ? 0u : attention_cluster_ctas(m->cfg.q_heads, m->cfg.kv_heads);
 }
 
 static stark_b200_status dense_reset(Model *m) {

@@ -111,7 +111,7 @@ struct Model {
     uint32_t *attn_counters = nullptr;
     float *partial_max = nullptr;
     uint32_t *partial_index = nullptr;
-    uint32_t attn_splits = 1;
+    uint32_t attn_splits = 1, attn_cluster = 0;
     cudaGraphExec_t step_graph = nullptr, ingest_graph = nullptr;
     // persistent-kernel path (STARK_B200_MEGA=1)
     bool use_mega = false;

@@ -83,6 +83,7 @@ stark_b200_status issue_draft_step(Model *m) {
     at.q_heads = c.q_heads;
     at.kv_heads = c.kv_heads;
     at.splits = m->attn_splits;
+    at.cluster = m->attn_cluster;
     at.scratch = m->attn_scratch;
     at.counters = m->attn_counters;
     at.error_word = ctx->error_word;

@@ -18,10 +18,14 @@ namespace {
 // row exists (104 KB of shared memory instead of 70 KB).
 // MINB: CTAs per SM the register allocation is sized for (5: at most 96 registers, so that a CTA fits beside
 // two resident 320-thread matvec CTAs at 80; 4: up to 128).
-template <int NBUF, int MINB>
+// CLUSTER: the splits of a head are a cluster and merge through distributed shared memory.  The last arriver's way -- partials to
+// memory, a fence, a counter, the partials back -- took 4.8 of the kernel's 10.2 us (8b shape, 4 100 rows; 4.5 of 7.7 behind 500 rows
+// of the 0.6b shape).
+template <int NBUF, int MINB, bool CLUSTER>
 __global__ void __launch_bounds__(kAttnThreads, MINB) attention_decode_kernel(const AttnParams p) {
     extern __shared__ __align__(128) uint8_t attn_smem[];
     __shared__ uint32_t is_last;
+    if (CLUSTER) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     pdl_launch_dependents();
     const uint32_t tid = threadIdx.x;
     const uint32_t split = blockIdx.x, h = blockIdx.y;
@@ -35,7 +39,8 @@ __global__ void __launch_bounds__(kAttnThreads, MINB) attention_decode_kernel(co
     // every kernel launches its dependents at once, so several later kernels can be resident and waiting
     // while the writer of `position` is still running: the position is read again after the wait and
     // the fetch repeated if it moved.
-    const AttnShared sm = carve_attn_shared(attn_smem, NBUF);
+    AttnShared sm = carve_attn_shared(attn_smem, NBUF);
+    if (CLUSTER) sm.stats = reinterpret_cast<float2 *>(sm.recv + p.gqa * kHeadDim + 16u);
     AttnPrefetch pf;
     attention_prefetch<NBUF>(p, split, h, __ldcg(&p.state->position), sm, tid, pf);
     pdl_wait();
@@ -43,13 +48,19 @@ __global__ void __launch_bounds__(kAttnThreads, MINB) attention_decode_kernel(co
         trace_min(&p.trace->ready);
         trace_max(&p.trace->ready_last);
     }
+    const AttnRows rows = attention_rows(p, h, tid);
     const uint32_t pos = __ldcg(&p.state->position);
     if (pos != pf.pos) {  // uniform across the CTA
         cp_async_wait<0>();
         __syncthreads();
         attention_prefetch<NBUF>(p, split, h, pos, sm, tid, pf);
     }
-    attention_partial<0, kAttnThreads, NBUF>(p, split, h, pos, sm, tid, pf);
+    attention_partial<0, kAttnThreads, NBUF, CLUSTER>(p, split, h, pos, sm, tid, pf, rows);
+    if constexpr (CLUSTER) {
+        attention_cluster_merge(p, split, h, sm, tid);
+        if (tid == 0 && p.trace) trace_max(&p.trace->end);
+        return;
+    }
     if (tid == 0) {
         const uint32_t prev = atomicAdd(&p.counters[h], 1u);
         is_last = prev == p.splits - 1u;
@@ -414,6 +425,40 @@ size_t attention_scratch_floats(uint32_t q_heads, uint32_t kv_heads, uint32_t sp
     return (size_t)q_heads * splits * (kHeadDim + 2u);
 }
 
+static cudaLaunchConfig_t attention_cluster_config(uint32_t gqa) {
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kAttnThreads);
+    cfg.dynamicSmemBytes = attn_shared_bytes(3u) + attn_cluster_bytes(gqa);
+    return cfg;
+}
+
+// The most CTAs (16 to 8) whose clusters, one for every head, the device holds at once with one CTA an SM -- the room the matvec before them
+// leaves: the smallest GPC decides.  Clusters of 16 on the 8b shape wait for that matvec to end (11.5 us against 10.2 through the
+// scratch).  64 to 148 CTAs in all: with fewer the cache is read by too few SMs.
+uint32_t attention_cluster_ctas(uint32_t q_heads, uint32_t kv_heads) {
+    if (kv_heads == 0 || q_heads % kv_heads != 0 || q_heads / kv_heads > (uint32_t)kMaxGqa) return 0u;
+    static SmemOptIn once;
+    const auto kernel = attention_decode_kernel<3, 5, true>;
+    if (ensure_dynamic_smem(kernel, 120 * 1024, once) != STARK_B200_OK) return 0u;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
+    for (uint32_t ctas = 16u; ctas >= 8u; --ctas) {
+        if (kv_heads * ctas > 148u || kv_heads * ctas < 64u) continue;
+        cudaLaunchConfig_t cfg = attention_cluster_config(q_heads / kv_heads);
+        cfg.gridDim = dim3(ctas, kv_heads);
+        cfg.dynamicSmemBytes = std::max<size_t>(cfg.dynamicSmemBytes, 115u * 1024u);  // no two to an SM
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = ctas;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) cudaGetLastError();
+        else if (clusters >= (int)kv_heads) return ctas;
+    }
+    return 0u;
+}
+
 stark_b200_status attention_decode_launch(const AttnArgs &a, cudaStream_t stream) {
     if (!a.qkv || !a.out || !a.kv.keys || !a.kv.values || !a.block_table || !a.state || !a.scratch || !a.counters)
         return STARK_B200_INVALID_ARGUMENT;
@@ -443,8 +488,24 @@ stark_b200_status attention_decode_launch(const AttnArgs &a, cudaStream_t stream
     const uint32_t bufs = tunables().attn_bufs;  // tile pairs in flight per CTA
     const bool wide = tunables().attn_regs >= 128u;
     using Kernel = void (*)(const AttnParams);
-    static const Kernel kernels[2][2] = {{attention_decode_kernel<2, 5>, attention_decode_kernel<2, 4>},
-                                         {attention_decode_kernel<3, 5>, attention_decode_kernel<3, 4>}};
+    if (a.cluster) {
+        p.splits = a.cluster;
+        cudaLaunchConfig_t cfg = attention_cluster_config(a.q_heads / a.kv_heads);
+        cfg.gridDim = dim3(a.cluster, a.kv_heads);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = a.cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = a.pdl ? 2 : 1;
+        SB_CUDA(cudaLaunchKernelEx(&cfg, attention_decode_kernel<3, 5, true>, (const AttnParams)p));
+        return STARK_B200_OK;
+    }
+    static const Kernel kernels[2][2] = {{attention_decode_kernel<2, 5, false>, attention_decode_kernel<2, 4, false>},
+                                         {attention_decode_kernel<3, 5, false>, attention_decode_kernel<3, 4, false>}};
     static SmemOptIn once[2][2];
     const uint32_t bi = bufs == 2u ? 0u : 1u, wi = wide ? 1u : 0u;
     const uint32_t smem = attn_shared_bytes(bi ? 3u : 2u);

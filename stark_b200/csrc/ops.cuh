@@ -50,7 +50,9 @@ struct AttnArgs {
     uint32_t *error_word;
     TraceSlot *trace;
     bool pdl;
+    uint32_t cluster;         // CTAs of a cluster that is a KV head's splits (attention_cluster_ctas); 0: `splits` CTAs through the scratch
 };
+uint32_t attention_cluster_ctas(uint32_t q_heads, uint32_t kv_heads);
 stark_b200_status attention_decode_launch(const AttnArgs &a, cudaStream_t stream);
 size_t attention_scratch_floats(uint32_t q_heads, uint32_t kv_heads, uint32_t splits);
 

@@ -251,3 +251,28 @@ def test_a_peer_that_never_answers_fences_the_handle_and_nothing_else():
     fresh.prefill(S.prompt(cfg, 5, seed=1))
     assert np.isfinite(fresh.logits()).all() and take_device_error() == 0
     fresh.close()
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(8, 8), (16, 8), (24, 8), (64, 8), (18, 9)])
+def test_splits_of_a_cluster_match_splits_through_memory(q_heads, kv_heads):
+    """Decode attention whose splits merge through distributed shared memory against the form that leaves partials in memory: one to
+    eight heads a group, shares of the outputs that do not divide, fewer pages than splits, page borders, a context of several
+    pages a split.  The same products; sums over keys and splits in another order."""
+    from stark_b200.engine import DenseModel
+    from stark_b200.ops import take_device_error
+    cfg = dict(S.CONFIGS["tiny"], layers=2, hidden=256, inter=128, q_heads=q_heads, kv_heads=kv_heads, vocab=512)
+    w = S.dense_weights(cfg, seed=q_heads, zero_point=7.5)
+    ids, seen = S.prompt(cfg, 2100, seed=6), []
+    model = DenseModel.load(cfg, w, context_tokens=2200)
+    for splits in (13, 0):
+        model.recapture(attn_splits=splits)
+        model.reset()
+        got, at = [], 0
+        for upto in (1, 63, 64, 65, 700, 2100):
+            model.prefill(ids[at:upto])
+            got.append(model.logits_bf16().copy())
+            at = upto
+        seen.append(got)
+    assert take_device_error() == 0
+    for through_memory, cluster in zip(*seen):
+        assert_logits_accepted(through_memory, cluster)
