@@ -153,6 +153,11 @@ stark_b200_status model_set_vector(Model *m, uint32_t layer, uint32_t which, con
     }
     if (layer >= m->layers.size()) return STARK_B200_INVALID_ARGUMENT;  // layers, then the draft head's layer
     auto &L = m->layers[layer];
+    if (which == STARK_B200_VEC_Q_NORM || which == STARK_B200_VEC_K_NORM) {
+        float top = 0.0f;
+        for (uint32_t i = 0; i < count; ++i) top = std::max(top, std::isfinite(data[i]) ? fabsf(data[i]) : INFINITY);
+        (which == STARK_B200_VEC_Q_NORM ? L.q_norm_top : L.k_norm_top) = top;
+    }
     switch (which) {
         case STARK_B200_VEC_ATTN_NORM: return upload_norm(&L.attn_norm, &L.attn_norm_b16, data, count);
         case STARK_B200_VEC_MLP_NORM: return upload_norm(&L.mlp_norm, &L.mlp_norm_b16, data, count);

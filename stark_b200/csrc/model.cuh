@@ -17,6 +17,7 @@ struct ModelLayer {
     QMatrix *o_rows = nullptr, *down_rows = nullptr;
     float *attn_norm = nullptr, *mlp_norm = nullptr, *q_norm = nullptr, *k_norm = nullptr;
     uint16_t *attn_norm_b16 = nullptr, *mlp_norm_b16 = nullptr;  // the norm weights rounded to bf16, as the kernels use them
+    float q_norm_top = 0.0f, k_norm_top = 0.0f;  // the head norms' largest weights, 0: none
     KvLayer kv{nullptr, nullptr};
 };
 

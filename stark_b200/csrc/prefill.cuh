@@ -89,6 +89,9 @@ struct PrefillAttnArgs {
     // Pages the cache arrays hold (the extent of the tensor maps): with it, passes of more than 16 rows run on the
     // tcgen05 tensor cores (prefill_attention_tc.cu); 0 keeps them on the mma.sync kernel.
     uint32_t num_blocks = 0;
+    // A bound of |q . k| * scale over all rows and keys (0: none known), as per-head norms give one: the tcgen05 form then looks at the
+    // keys once instead of twice.
+    float score_bound = 0.0f;
     uint32_t whole_heads = 0;  // query heads over all ranks (0: q_heads), as whole_rows above
 };
 constexpr uint32_t kPrefillAttnMaxSplits = 64;

@@ -3,20 +3,25 @@
 // 1/sqrt(d), softmax in f32, probabilities into the second product as bf16 hi + lo, output rounded to bf16), in the
 // shape the tensor core wants.
 //
-// One CTA owns 128 rows of one query head and walks the keys in steps of 128 (two pages of the cache) TWICE:
-//   pass 1   S = Q K^T per step, only to find every row's maximum;
+// One CTA owns 128 rows of one query head and walks the keys in steps of 128 (two pages of the cache), in two passes:
+//   pass 1   S = Q K^T per step, only to find every row's maximum; left out where the head norms bound the scores (PrefillAttnArgs)
 //   pass 2   S again, P = exp2(S - max) (already final: no accumulator is ever rescaled), O += P V.
 // The second look at the keys costs a quarter more tensor-core work and removes the read-modify-write of the output
 // accumulator that an online softmax needs whenever a maximum moves.  Roles:
 //   warps 0-7   softmax: thread = row (tensor-memory lane) x half of the step's keys; tcgen05.ld of S in 32-column
-//               pieces, mask by the row's causal limit, maximum (pass 1) or exp2 / row sum / bf16 hi + lo written as
-//               the K-major, 128-byte swizzled A operand of the second product (pass 2); at the end the read-out of O
+//               pieces, mask by the row's causal limit, maximum (pass 1) or exp2 / row sum / bf16 hi + lo stored to tensor
+//               memory, the A operand of the second product (pass 2); at the end the read-out of O
 //   warp 8      one thread: TMA loads -- Q once, then per step the K tile (and in pass 2 the V tile) as four
 //               [64 keys x 64 dims] boxes straight from the paged cache
-//   warp 9      owns tensor memory (S twice, so that step j + 1 is multiplied while step j is exponentiated, and O);
+//   warp 9      owns tensor memory (S twice, so that step j + 1 is multiplied while step j is exponentiated, O and P);
 //               one thread issues the MMAs: S = Q K^T with both operands K-major, O += P V with V as an MN-major
 //               operand (its rows are keys, the contraction index), and commits them to the barriers
 // Every wait is bounded; a wait that runs out sets the error word, the CTA drains and frees its tensor memory.
+//
+// What bounds it: the chain of a step through the softmax warps (about nine instructions for two probabilities, two warps a scheduler),
+// beside 1 536 tensor-core cycles.  4 096 rows of the 8b shape, a layer: 571 000 cycles with P in shared memory and two passes, 524 000 with P in
+// tensor memory, masks out of line and sums in four chains, 515 000 with paired f32 instructions, 398 000 in one pass (336 -> 234 us).
+// Three stages instead of two and four score tiles in pass 1 changed nothing alone.
 //
 // Few rows over many keys (SPLIT): 16 heads of one row block are 16 CTAs that walk the whole cache one after another.  The
 // keys are then divided among the CTAs of a cluster: they exchange the rows' maxima between the passes, so that every CTA's
@@ -40,10 +45,13 @@ constexpr uint32_t kBox = 64u * 128u;       // [64 rows][64 elements] bf16 in 12
 constexpr uint32_t kBlock = 2u * kBox;      // 128 rows x 64 elements: 16 KB
 constexpr uint32_t kOperand = 2u * kBlock;  // 128 x 128: 32 KB
 constexpr uint32_t kSoftmaxWarps = 8, kTcThreads = (kSoftmaxWarps + 2u) * 32u;
-// shared memory: Q | K, two stages | V, two stages | P hi | P lo | barriers (256 B) | exchange words [2][128] f32
-constexpr uint32_t kQOff = 0, kKOff = kOperand, kVOff = 3u * kOperand, kPOff = 5u * kOperand, kBarOff = 7u * kOperand;
-constexpr uint32_t kTcSmem = 7u * kOperand + 2048u /* barriers, exchange words */ + 1024u /* alignment */;
-constexpr uint32_t kTcTmemColumns = 512;  // S twice (2 x 128) and O (128); allocations are powers of two
+// shared memory: Q | K, three stages | V, three stages | barriers (512 B) | exchange words [2][128] f32
+constexpr uint32_t kDepth = 3;
+constexpr uint32_t kQOff = 0, kKOff = kOperand, kVOff = kKOff + kDepth * kOperand, kBarOff = kVOff + kDepth * kOperand;
+constexpr uint32_t kSumsOff = kVOff + kOperand;  // SPLIT, at the end: the row sums, behind the shares of O
+constexpr uint32_t kTcSmem = kBarOff + 2048u /* barriers, exchange words */ + 1024u /* alignment */;
+constexpr uint32_t kTcTmemColumns = 512;  // S twice (2 x 128), O (128), P as pairs of bf16: 64 columns hi, 64 lo
+constexpr uint32_t kPColumn = 384;
 // D f32, A and B bf16, M 128, N 128; the second product takes B (V) MN-major
 constexpr uint32_t kIdescS = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t kIdescPV = kIdescS | (1u << 16);
@@ -54,14 +62,41 @@ __device__ inline float ex2_approx(float x) {
     return y;
 }
 
+// Two f32 operations in one instruction, each rounded as the single one.
+__device__ inline float2 fma_pair(float2 a, float2 b, float2 c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)), "l"(*reinterpret_cast<uint64_t *>(&c)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+__device__ inline float2 add_pair(float2 a, float2 b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)));
+    return *reinterpret_cast<float2 *>(&d);
+}
+
+// A bound (in powers of two) up to which it may stand in for a row's maximum: probabilities then lie above 2^-96, a row's largest too,
+// so that every one that counts beside it is a normal f32 -- the same relative precision as behind the maximum itself.
+constexpr float kMostBound = 48.0f;
+
 struct TcAttnParams {
     uint16_t *out;
     const int32_t *block_table;
     uint32_t m, first_pos, q_heads, kv_heads, gqa, num_blocks;
     float scale_log2;  // log2(e) / sqrt(d)
+    float bound;       // no score times scale_log2 is larger (0: unknown); it stands in for the rows' maxima
     uint32_t *error_word;
     uint32_t stop_after;  // 0 whole kernel; 1 set-up and tensor memory only; 2 pass 1 only (no MN-major operand)
 };
+
+// Scores of keys past `pos` become -inf: probabilities of exactly zero.  Only steps on the diagonal have any; the others pay one branch.
+__device__ __forceinline__ void hide_keys(uint32_t (&v)[32], uint32_t key0, uint32_t pos) {
+    if (key0 + 31u <= pos) return;
+#pragma unroll
+    for (uint32_t i = 0; i < 32u; ++i)
+        if (key0 + i > pos) v[i] = 0xff800000u;
+}
 
 constexpr uint32_t kPartPitch = 128u + 4u;  // floats between the rows of a CTA's share of O, in place of the K and V stages
 
@@ -72,13 +107,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     extern __shared__ uint8_t tc_smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023u) & ~(uintptr_t)1023u);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kBarOff);
-    uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7;
-    uint64_t *s_full = bars + 9, *s_free = bars + 11, *p_full = bars + 13, *p_free = bars + 14, *o_full = bars + 15;
-    uint64_t *a_full = bars + 16, *a_empty = bars + 20;  // pass 1: the K and V stages together are a ring of four K tiles
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 24);
+    uint64_t *q_full = bars, *s_full = bars + 1, *s_free = bars + 3, *p_full = bars + 5, *p_free = bars + 6, *o_full = bars + 7;
+    uint64_t *m_full = bars + 8, *m_free = bars + 12;  // pass 1: all of tensor memory is four score tiles
+    uint64_t *k_full = bars + 16, *k_empty = k_full + kDepth, *v_full = k_empty + kDepth, *v_empty = v_full + kDepth;
+    uint64_t *a_full = v_empty + kDepth, *a_empty = a_full + 2u * kDepth;  // pass 1: the K and V stages together are one ring of K tiles
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(a_empty + 2u * kDepth);
     volatile uint32_t *abort_flag = tmem_slot + 1;
-    float *exchange = reinterpret_cast<float *>(smem + kBarOff + 256u);  // what the two warps of a row tell each other
-    float *part_sums = reinterpret_cast<float *>(smem + kPOff);  // SPLIT: the row sums [2][128], at the end
+    float *exchange = reinterpret_cast<float *>(smem + kBarOff + 512u);  // what the two warps of a row tell each other
+    float *part_sums = reinterpret_cast<float *>(smem + kSumsOff);  // SPLIT: the row sums [2][128], at the end
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t head = blockIdx.x, kvh = head / p.gqa;
@@ -88,19 +124,25 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     const uint32_t all_steps = (p.first_pos + last_row) / 128u + 1u;
     const uint32_t split = SPLIT ? gridDim.z : 1u, rank = SPLIT ? blockIdx.z : 0u;  // the cluster is the grid's z
     const uint32_t step0 = all_steps * rank / split, steps = all_steps * (rank + 1u) / split - step0;  // possibly none
-    const uint32_t passes = p.stop_after == 2u ? 1u : 2u;
+    const uint32_t passes = p.stop_after == 2u ? 1u : 2u, first_steps = p.bound > 0.0f ? 0u : steps;  // of pass 1
 
     if (tid == 0) {
         mbar_init(q_full, 1);
         for (uint32_t s = 0; s < 2; ++s) {
-            mbar_init(&k_full[s], 1);
-            mbar_init(&k_empty[s], 1);
-            mbar_init(&v_full[s], 1);
-            mbar_init(&v_empty[s], 1);
             mbar_init(&s_full[s], 1);
             mbar_init(&s_free[s], kSoftmaxWarps);
         }
         for (uint32_t s = 0; s < 4; ++s) {
+            mbar_init(&m_full[s], 1);
+            mbar_init(&m_free[s], kSoftmaxWarps);
+        }
+        for (uint32_t s = 0; s < kDepth; ++s) {
+            mbar_init(&k_full[s], 1);
+            mbar_init(&k_empty[s], 1);
+            mbar_init(&v_full[s], 1);
+            mbar_init(&v_empty[s], 1);
+        }
+        for (uint32_t s = 0; s < 2u * kDepth; ++s) {
             mbar_init(&a_full[s], 1);
             mbar_init(&a_empty[s], 1);
         }
@@ -118,7 +160,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     pdl_launch_dependents();
     pdl_wait();  // the rows and the cache rows appended for them
     // the maxima are the softmax warps' business: the other two arrive ahead and collect the barrier at their end
-    const bool bystander = SPLIT && warp >= kSoftmaxWarps;
+    const bool bystander = SPLIT && warp >= kSoftmaxWarps && !(p.bound > 0.0f);
     if (bystander) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     auto give_up = [&]() {
         *abort_flag = 1;
@@ -147,16 +189,16 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             };
             uint32_t ks = 0, kph = 1, vs = 0, vph = 1;  // a fresh barrier passes a wait on parity 1
             bool ok = true;
-            {   // pass 1: K tiles only, four in flight
+            {   // pass 1: K tiles only
                 uint32_t as = 0, aph = 1;
-                for (uint32_t j = 0; j < steps && ok; ++j) {
+                for (uint32_t j = 0; j < first_steps && ok; ++j) {
                     if (!(ok = mbar_wait_bounded(&a_empty[as], aph, abort_flag))) break;
                     load_tile(smem + kKOff + as * kOperand, &k_map, page_row(2u * (step0 + j)), page_row(2u * (step0 + j) + 1u), &a_full[as]);
-                    if (++as == 4u) as = 0, aph ^= 1u;
+                    if (++as == 2u * kDepth) as = 0, aph ^= 1u;
                 }
                 // pass 2 loads into the same memory: every stage's last pass-1 tile must have been multiplied
-                for (uint32_t s = 0; s < 4u && ok && passes == 2u; ++s) {
-                    const uint32_t uses = steps > s ? (steps - s + 3u) / 4u : 0u;
+                for (uint32_t s = 0; s < 2u * kDepth && ok && passes == 2u; ++s) {
+                    const uint32_t uses = first_steps > s ? (first_steps - s + 2u * kDepth - 1u) / (2u * kDepth) : 0u;
                     if (uses) ok = mbar_wait_bounded(&a_empty[s], (uses - 1u) & 1u, abort_flag);
                 }
             }
@@ -165,11 +207,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     const uint32_t y0 = page_row(2u * (step0 + j)), y1 = page_row(2u * (step0 + j) + 1u);
                     if (!(ok = mbar_wait_bounded(&k_empty[ks], kph, abort_flag))) break;
                     load_tile(smem + kKOff + ks * kOperand, &k_map, y0, y1, &k_full[ks]);
-                    if (++ks == 2u) ks = 0, kph ^= 1u;
+                    if (++ks == kDepth) ks = 0, kph ^= 1u;
                     if (pass == 1u) {
                         if (!(ok = mbar_wait_bounded(&v_empty[vs], vph, abort_flag))) break;
                         load_tile(smem + kVOff + vs * kOperand, &v_map, y0, y1, &v_full[vs]);
-                        if (++vs == 2u) vs = 0, vph ^= 1u;
+                        if (++vs == kDepth) vs = 0, vph ^= 1u;
                     }
                 }
             }
@@ -181,11 +223,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             bool ok = mbar_wait_bounded(q_full, 0, abort_flag);
             uint32_t ks = 0, kph = 0, vs = 0, vph = 0, g = 0;  // g counts score tiles: buffer g & 1
             const uint32_t q_addr = smem_u32(smem + kQOff);
-            const uint32_t ring = 4u;  // pass 1; pass 2 below passes 2
-            auto scores = [&](uint64_t *full, uint64_t *empty, uint32_t slots) {
-                const uint32_t b = g & 1u, use = g >> 1;
+            auto scores = [&](uint64_t *full, uint64_t *empty, uint32_t slots, uint64_t *tile_full, uint64_t *tile_free, uint32_t tiles) {
+                const uint32_t b = g % tiles, use = g / tiles;
                 ok = ok && mbar_wait_bounded(&full[ks], kph, abort_flag) &&
-                     mbar_wait_bounded(&s_free[b], (use & 1u) ^ 1u, abort_flag);  // the softmax warps are done with use - 1
+                     mbar_wait_bounded(&tile_free[b], (use & 1u) ^ 1u, abort_flag);  // the softmax warps are done with use - 1
                 if (!ok) return;
                 tc_fence_after();
                 const uint32_t k_addr = smem_u32(smem + kKOff + ks * kOperand);
@@ -196,16 +237,18 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                              i != 0u ? 1u : 0u);
                 }
                 umma_commit(&empty[ks]);
-                umma_commit(&s_full[b]);
+                umma_commit(&tile_full[b]);
                 if (++ks == slots) ks = 0, kph ^= 1u;
                 ++g;
             };
-            for (uint32_t j = 0; j < steps && ok; ++j) scores(a_full, a_empty, ring);
-            ks = 0, kph = 0;
+            for (uint32_t j = 0; j < first_steps && ok; ++j) scores(a_full, a_empty, 2u * kDepth, m_full, m_free, 4u);
+            ks = 0, kph = 0, g = 0;
             if (passes == 2u) {
-                const uint32_t ph_addr = smem_u32(smem + kPOff), pl_addr = ph_addr + kOperand;
+                for (uint32_t b = 0; b < 4u && ok; ++b)  // O and P take the place of score tiles that have been read
+                    if (first_steps > b) ok = mbar_wait_bounded(&m_free[b], ((first_steps - b + 3u) / 4u - 1u) & 1u, abort_flag);
+                tc_fence_after();
                 for (uint32_t j = 0; j <= steps && ok; ++j) {
-                    if (j < steps) scores(k_full, k_empty, 2u);  // step j is multiplied while step j - 1 is exponentiated
+                    if (j < steps) scores(k_full, k_empty, kDepth, s_full, s_free, 2u);  // step j is multiplied while step j - 1 is exponentiated
                     if (j == 0u || !ok) continue;
                     const uint32_t t = j - 1u;
                     ok = mbar_wait_bounded(p_full, t & 1u, abort_flag) && mbar_wait_bounded(&v_full[vs], vph, abort_flag);
@@ -215,13 +258,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
 #pragma unroll
                     for (uint32_t i = 0; i < 8u; ++i) {  // 16 keys a step
                         const uint64_t vdesc = smem_desc_sw128_mn(v_addr + i * 2048u, kBlock);
-                        const uint32_t at = (i >> 2) * kBlock + (i & 3u) * 32u;
-                        umma_f16(tmem_base + 256u, smem_desc_sw128(ph_addr + at), vdesc, kIdescPV, (t | i) != 0u ? 1u : 0u);
-                        umma_f16(tmem_base + 256u, smem_desc_sw128(pl_addr + at), vdesc, kIdescPV, 1u);
+                        umma_f16_ts(tmem_base + 256u, tmem_base + kPColumn + 8u * i, vdesc, kIdescPV, (t | i) != 0u ? 1u : 0u);
+                        umma_f16_ts(tmem_base + 256u, tmem_base + kPColumn + 64u + 8u * i, vdesc, kIdescPV, 1u);
                     }
                     umma_commit(&v_empty[vs]);
                     umma_commit(p_free);
-                    if (++vs == 2u) vs = 0, vph ^= 1u;
+                    if (++vs == kDepth) vs = 0, vph ^= 1u;
                 }
             }
             if (!ok) give_up();
@@ -238,9 +280,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         float mrow = -INFINITY;
         uint32_t g = 0;
         bool ok = true;
-        for (uint32_t j = 0; j < steps && ok; ++j, ++g) {
-            const uint32_t b = g & 1u;
-            if (!(ok = mbar_wait_bounded(&s_full[b], (g >> 1) & 1u, abort_flag))) break;
+        for (uint32_t j = 0; j < first_steps && ok; ++j) {
+            const uint32_t b = j & 3u;
+            if (!(ok = mbar_wait_bounded(&m_full[b], (j >> 2) & 1u, abort_flag))) break;
             tc_fence_after();
             uint32_t v[2][32];
 #pragma unroll
@@ -248,83 +290,79 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
 #pragma unroll
             for (uint32_t c = 0; c < 2u; ++c) {
                 tmem_ld_wait_32(v[c]);
-                const uint32_t key0 = (step0 + j) * 128u + col0 + 32u * c;
-                float mx = -INFINITY;
-                if (key0 + 31u <= pos) {  // the row sees the whole piece
+                hide_keys(v[c], (step0 + j) * 128u + col0 + 32u * c, pos);
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(v[c][i]));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (key0 + i <= pos) mx = fmaxf(mx, __uint_as_float(v[c][i]));
-                }
-                mrow = fmaxf(mrow, mx * p.scale_log2);  // the scale is positive: it commutes with the maximum
+                for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[c][i]));
+                mrow = fmaxf(mrow, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);  // the scale is positive: it commutes with the maximum
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&s_free[b]);
+            if (lane == 0) mbar_arrive(&m_free[b]);
         }
         // the row's maximum over both halves of the keys
-        exchange[half * 128u + r] = mrow;
-        if constexpr (SPLIT) {
-            __syncwarp();
-            thin_cluster_sync();
-            mrow = thin_fold(&exchange[r], split, mrow, [](float a, float b) { return fmaxf(a, b); });
+        if (p.bound > 0.0f) {
+            mrow = p.bound;
         } else {
-            named_bar_sync(1, kSoftmaxWarps * 32u);
-            mrow = fmaxf(mrow, exchange[(half ^ 1u) * 128u + r]);
-            named_bar_sync(1, kSoftmaxWarps * 32u);  // everybody has read: the words are free for the row sums
+            exchange[half * 128u + r] = mrow;
+            if constexpr (SPLIT) {
+                __syncwarp();
+                thin_cluster_sync();
+                mrow = thin_fold(&exchange[r], split, mrow, [](float a, float b) { return fmaxf(a, b); });
+            } else {
+                named_bar_sync(1, kSoftmaxWarps * 32u);
+                mrow = fmaxf(mrow, exchange[(half ^ 1u) * 128u + r]);
+                named_bar_sync(1, kSoftmaxWarps * 32u);  // everybody has read: the words are free for the row sums
+            }
         }
         float l = 0.0f;
+        float2 sums[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(-mrow, -mrow), minus1 = make_float2(-1.0f, -1.0f);
         if (passes == 2u) {
-            uint8_t *p_hi = smem + kPOff + half * kBlock + r * 128u, *p_lo = p_hi + kOperand;  // key block `half` of the row
             for (uint32_t j = 0; j < steps && ok; ++j, ++g) {
                 const uint32_t b = g & 1u;
                 if (!(ok = mbar_wait_bounded(&s_full[b], (g >> 1) & 1u, abort_flag))) break;
                 tc_fence_after();
-                uint32_t v[2][32];
+                uint32_t v[2][32], hi[2][16], lo[2][16];
                 tmem_ld_32x32_issue(tmem_base + lanes + b * 128u + col0, v[0]);
                 tmem_ld_32x32_issue(tmem_base + lanes + b * 128u + col0 + 32u, v[1]);
+                tmem_ld_wait_32(v[0]);
+                tmem_ld_wait_32(v[1]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_free[b]);
 #pragma unroll
                 for (uint32_t c = 0; c < 2u; ++c) {
-                    if (!ok) break;
-                    uint32_t hi[16], lo[16];
-                    tmem_ld_wait_32(v[c]);
-                    const uint32_t key0 = (step0 + j) * 128u + col0 + 32u * c;
-                    const bool whole = key0 + 31u <= pos;
+                    hide_keys(v[c], (step0 + j) * 128u + col0 + 32u * c, pos);
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
                         // exp2 of a non-positive argument: the hardware approximation is good to two units of an f32's
                         // last place, far inside what the bf16 pair keeps
-                        float e0 = ex2_approx(fmaf(__uint_as_float(v[c][i]), p.scale_log2, -mrow));
-                        float e1 = ex2_approx(fmaf(__uint_as_float(v[c][i + 1]), p.scale_log2, -mrow));
-                        if (!whole) {
-                            if (key0 + i > pos) e0 = 0.0f;
-                            if (key0 + i + 1 > pos) e1 = 0.0f;
-                        }
-                        l += e0;
-                        l += e1;
-                        split_bf16x2(e0, e1, hi[i >> 1], lo[i >> 1]);
-                    }
-                    // the previous step's second product must have read P before it is overwritten
-                    if (c == 0u && !(ok = mbar_wait_bounded(p_free, (j & 1u) ^ 1u, abort_flag))) break;
-                    // 32 keys = four 16-byte chunks of the row's 128-byte line
-#pragma unroll
-                    for (uint32_t q = 0; q < 4u; ++q) {
-                        const uint32_t at = ((c * 4u + q) ^ (r & 7u)) << 4;
-                        *reinterpret_cast<uint4 *>(p_hi + at) = make_uint4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
-                        *reinterpret_cast<uint4 *>(p_lo + at) = make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
+                        const float2 x = fma_pair(make_float2(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), scale2, shift2);
+                        const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+                        sums[i >> 1 & 1] = add_pair(sums[i >> 1 & 1], e);
+                        const uint32_t h = f32x2_to_bf16x2(e.x, e.y);  // hi + lo: two roundings to nearest
+                        const float2 rest = fma_pair(make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus1, e);
+                        hi[c][i >> 1] = h;
+                        lo[c][i >> 1] = f32x2_to_bf16x2(rest.x, rest.y);
                     }
                 }
-                proxy_fence_async();  // the tensor core reads shared memory through the async proxy
+                // the previous step's second product must have read P before it is overwritten; the warp goes on as one
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(p_free, (j & 1u) ^ 1u, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (uint32_t c = 0; c < 2u; ++c) {  // 32 keys = 16 columns of pairs
+                    tmem_st_32x16(tmem_base + lanes + kPColumn + half * 32u + c * 16u, hi[c]);
+                    tmem_st_32x16(tmem_base + lanes + kPColumn + 64u + half * 32u + c * 16u, lo[c]);
+                }
+                tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&s_free[b]);
-                    mbar_arrive(p_full);
-                }
+                if (lane == 0) mbar_arrive(p_full);
             }
-            // the row's sum over both halves, in key order
+            l = (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
+            // the row's sum over both halves
             if constexpr (!SPLIT) {
                 exchange[half * 128u + r] = l;
                 named_bar_sync(1, kSoftmaxWarps * 32u);
@@ -437,6 +475,7 @@ stark_b200_status prefill_attention_tc_launch(const PrefillAttnArgs &a, cudaStre
     p.gqa = a.q_heads / a.kv_heads;
     p.num_blocks = a.num_blocks;
     p.scale_log2 = a.scale * 1.4426950408889634f;
+    p.bound = tunables().prefill_attn_tc == 1u && a.score_bound > 0.0f && a.score_bound * 1.4426950408889634f <= kMostBound ? a.score_bound * 1.4426950408889634f : 0.0f;
     p.error_word = ctx->error_word;
     p.stop_after = tunables().attn_tc_stop_after;
     // 77 rows behind 1 024 (16 heads, 28 layers): 2.87 ms with one CTA a row block, 2.72 with two, 2.50 with four, 2.86 with eight

@@ -208,6 +208,8 @@ stark_b200_status model_rows_pass(Model *m, const uint32_t *tokens_device, uint3
         pa.partials = m->rows_attn_partials;
         pa.max_splits = kPrefillAttnMaxSplits;
         pa.num_blocks = m->num_blocks;
+        // a normed head's norm is at most sqrt(dim) times its norm's largest weight; rotation keeps it; a hundredth for the roundings
+        pa.score_bound = 1.01f * scale * (float)kHeadDim * L.q_norm_top * L.k_norm_top;
         pa.whole_heads = c.q_heads * ranks;
         if ((st = prefill_attention_launch(pa, s)) != STARK_B200_OK) return st;
         if (tp && (st = gather(m->chunk_attn, attn_local, rows_region_attn(m), attn_width, rank * attn_local, attn_local,

@@ -296,3 +296,32 @@ def test_unpacked_weights_leave_the_same_bits(rows, hidden, q_heads, inter):
         _set("gemm_unpack", 1)
     assert take_device_error() == 0
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("gain,prefix,rows", [(1.0, 0, 200), (1.0, 900, 77), (1.6, 0, 641), (4.0, 0, 200)])
+def test_attention_in_one_pass_where_head_norms_bound_the_scores(gain, prefix, rows):
+    """Prompt attention with the norms' bound in the place of the rows' maxima against the two passes that find them: ragged row blocks,
+    keys on one CTA and on a cluster, weights near the largest bound that is used and beyond it (two passes on both sides)."""
+    from stark_b200.engine import DenseModel
+    from stark_b200.ops import take_device_error
+    from tests.test_model_gpu import assert_logits_accepted
+    cfg = dict(S.CONFIGS["small"], layers=2)
+    w = S.dense_weights(cfg, seed=12, zero_point=7.5)
+    for layer in w["layers"]:
+        layer["q_norm"], layer["k_norm"] = (gain * layer[k] / np.abs(layer[k]).max() for k in ("q_norm", "k_norm"))
+    model = DenseModel.load(cfg, w, context_tokens=prefix + rows + 8)
+    ids, got = S.prompt(cfg, prefix + rows + 1, seed=5), []
+    try:
+        for passes in (2, 1):
+            _set("prefill_attn_tc", passes)
+            model.reset()
+            if prefix:
+                model.prefill(ids[:prefix])
+            model.prefill(ids[prefix:])
+            got.append(model.logits_bf16().copy())
+    finally:
+        _set("prefill_attn_tc", 1)
+    assert take_device_error() == 0
+    if gain == 4.0:
+        assert np.array_equal(got[0], got[1])
+    assert_logits_accepted(got[0], got[1])
