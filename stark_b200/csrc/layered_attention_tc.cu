@@ -21,6 +21,7 @@
 #include "device_math.cuh"
 #include "layered.cuh"
 #include "layered_math.cuh"
+#include "softmax_tc.cuh"
 #include "tc05.cuh"
 #include "thin_tile.cuh"
 
@@ -28,23 +29,25 @@ namespace sb {
 
 namespace {
 
-constexpr uint32_t kKeys = kPageTokens;       // keys per step
-constexpr uint32_t kKeyBlock = kKeys * 128u;  // 64 keys x 64 elements: 8 KB
+constexpr uint32_t kPageBox = kPageTokens * 128u;  // 64 keys x 64 elements: 8 KB
 constexpr uint32_t kRowBlock = 128u * 128u;   // 128 rows x 64 elements: 16 KB
 constexpr uint32_t kSoftmaxWarps = 8, kThreads = (kSoftmaxWarps + 2u) * 32u;
 constexpr uint32_t kMaxKeyStages = 3, kValueStages = 2;
 constexpr uint32_t kMaxBlocks = 4;            // widths up to 256
 constexpr uint32_t kTail = 2048u;             // barriers, exchange words
-constexpr uint32_t kTmemColumns = 512, kOutColumn = 128;  // S twice (2 x 64), O from column 128 (up to 256)
+constexpr uint32_t kTmemColumns = 512;
 constexpr uint32_t kIdescBase = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
-constexpr uint32_t kIdescS = kIdescBase | ((kKeys >> 3) << 17);
+// Steps of one page: S twice (2 x 64 columns of tensor memory), O from column 128 (up to 256), P in shared memory.  Steps of two: S twice
+// (2 x 128), O (up to 128) and P (64 columns of pairs hi, 64 lo).
+template <uint32_t PAGES>
+struct Step {
+    static constexpr uint32_t kKeys = PAGES * kPageTokens, kBlock = PAGES * kPageBox;  // keys; bytes of 64 elements of all of them
+    static constexpr uint32_t kOutColumn = PAGES == 1u ? 128u : 256u, kPColumn = 384u;
+    static constexpr uint32_t kIdescS = kIdescBase | ((kKeys >> 3) << 17);
+};
 constexpr uint32_t kIdescPV = kIdescBase | (1u << 16);  // B (the values) MN-major; N is added at run time
 
-__device__ inline float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
+constexpr uint32_t kNoRow = 0x3fffffffu;  // past the end of every operand
 
 struct AttendTcParams {
     uint16_t *out;
@@ -60,21 +63,22 @@ struct AttendTcParams {
     uint32_t *error_word;
 };
 
-uint32_t tc_smem_bytes(uint32_t q_blocks, uint32_t v_blocks, uint32_t key_stages) {
-    return q_blocks * kRowBlock + key_stages * q_blocks * kKeyBlock + kValueStages * v_blocks * kKeyBlock + 2u * kRowBlock +
+uint32_t tc_smem_bytes(uint32_t pages, uint32_t q_blocks, uint32_t v_blocks, uint32_t key_stages) {
+    return q_blocks * kRowBlock + (key_stages * q_blocks + kValueStages * v_blocks) * pages * kPageBox + (pages == 1u ? 2u * kRowBlock : 0u) +
            kTail + 1024u;
 }
 
-template <bool SPLIT>
+template <bool SPLIT, uint32_t PAGES>
 __global__ void __launch_bounds__(kThreads, 1)
 attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                  const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap shared_map, const AttendTcParams p) {
+    using T = Step<PAGES>;
     extern __shared__ uint8_t attend_tc_smem[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(attend_tc_smem) + 1023u) & ~(uintptr_t)1023u);
     const uint32_t qb = p.own_blocks + p.shared_blocks, vb = p.value_blocks;
-    const uint32_t key_bytes = qb * kKeyBlock, value_bytes = vb * kKeyBlock;
+    const uint32_t key_bytes = qb * T::kBlock, value_bytes = vb * T::kBlock;
     uint8_t *q_smem = smem, *k_smem = q_smem + qb * kRowBlock, *v_smem = k_smem + p.key_stages * key_bytes;
-    uint8_t *p_smem = v_smem + kValueStages * value_bytes, *tail = p_smem + 2u * kRowBlock;
+    uint8_t *p_smem = v_smem + kValueStages * value_bytes, *tail = p_smem + (PAGES == 1u ? 2u * kRowBlock : 0u);
     uint64_t *bars = reinterpret_cast<uint64_t *>(tail);
     uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 4, *v_full = bars + 7, *v_empty = bars + 9;
     uint64_t *s_full = bars + 11, *s_free = bars + 13, *p_full = bars + 15, *p_free = bars + 16, *o_full = bars + 17;
@@ -86,7 +90,7 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     const uint32_t head = blockIdx.x, key_head = head / (p.heads / p.key_heads);
     const uint32_t row0 = (gridDim.y - 1u - blockIdx.y) * 128u;  // late row blocks read the most keys: first
     const uint32_t last_row = min(p.m, row0 + 128u) - 1u;
-    const uint32_t all_steps = (p.first_pos + last_row) / kKeys + 1u;
+    const uint32_t all_steps = (p.first_pos + last_row) / T::kKeys + 1u, pages = (p.first_pos + p.m - 1u) / kPageTokens + 1u;
     const uint32_t split = SPLIT ? gridDim.z : 1u, rank = SPLIT ? blockIdx.z : 0u;  // the cluster is the grid's z
     const uint32_t step0 = all_steps * rank / split, steps = all_steps * (rank + 1u) / split - step0;  // possibly none
     // SPLIT: this CTA's share of O [128][pitch] and of the row sums [2][128], at the end, when every operand has been read
@@ -136,21 +140,32 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
             bool ok = true;
             for (uint32_t pass = p.one_pass; pass < 2u && ok; ++pass) {
                 for (uint32_t j = 0; j < steps && ok; ++j) {
-                    const uint32_t page = (uint32_t)p.block_table[step0 + j], y = (page * p.key_heads + key_head) * kKeys;
+                    uint32_t page[PAGES], y[PAGES];
+#pragma unroll
+                    for (uint32_t i = 0; i < PAGES; ++i) {  // a page behind the last is read out of bounds: zeros
+                        const uint32_t at = PAGES * (step0 + j) + i;
+                        page[i] = at < pages ? (uint32_t)p.block_table[at] * kPageTokens : kNoRow;
+                        y[i] = at < pages ? page[i] * p.key_heads + key_head * kPageTokens : kNoRow;
+                    }
                     if (!(ok = mbar_wait_bounded(&k_empty[ks], kph, abort_flag))) break;
                     uint8_t *dst = k_smem + ks * key_bytes;
                     mbar_arrive_expect_tx(&k_full[ks], key_bytes);
-                    for (uint32_t b = 0; b < p.own_blocks; ++b)
-                        tma_load_2d(dst + b * kKeyBlock, &k_map, p.key_first + head * p.key_stride + b * 64u, y, &k_full[ks]);
-                    for (uint32_t b = 0; b < p.shared_blocks; ++b)
-                        tma_load_2d(dst + (p.own_blocks + b) * kKeyBlock, &shared_map, p.shared_first + b * 64u, page * kKeys, &k_full[ks]);
+#pragma unroll
+                    for (uint32_t i = 0; i < PAGES; ++i) {
+                        for (uint32_t b = 0; b < p.own_blocks; ++b)
+                            tma_load_2d(dst + b * T::kBlock + i * kPageBox, &k_map, p.key_first + head * p.key_stride + b * 64u, y[i], &k_full[ks]);
+                        for (uint32_t b = 0; b < p.shared_blocks; ++b)
+                            tma_load_2d(dst + (p.own_blocks + b) * T::kBlock + i * kPageBox, &shared_map, p.shared_first + b * 64u, page[i], &k_full[ks]);
+                    }
                     if (++ks == p.key_stages) ks = 0, kph ^= 1u;
                     if (pass == 1u) {
                         if (!(ok = mbar_wait_bounded(&v_empty[vs], vph, abort_flag))) break;
                         mbar_arrive_expect_tx(&v_full[vs], value_bytes);
-                        for (uint32_t b = 0; b < vb; ++b)
-                            tma_load_2d(v_smem + vs * value_bytes + b * kKeyBlock, &v_map,
-                                        p.value_first + head * p.value_stride + b * 64u, y, &v_full[vs]);
+#pragma unroll
+                        for (uint32_t i = 0; i < PAGES; ++i)
+                            for (uint32_t b = 0; b < vb; ++b)
+                                tma_load_2d(v_smem + vs * value_bytes + b * T::kBlock + i * kPageBox, &v_map,
+                                            p.value_first + head * p.value_stride + b * 64u, y[i], &v_full[vs]);
                         if (++vs == kValueStages) vs = 0, vph ^= 1u;
                     }
                 }
@@ -173,8 +188,8 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
                 for (uint32_t blk = 0; blk < qb; ++blk)
 #pragma unroll
                     for (uint32_t i = 0; i < 4u; ++i)  // 16 entries a step; 64 a block
-                        umma_f16(tmem_base + b * kKeys, smem_desc_sw128(q_addr + blk * kRowBlock + i * 32u),
-                                 smem_desc_sw128(k_addr + blk * kKeyBlock + i * 32u), kIdescS, (blk | i) != 0u ? 1u : 0u);
+                        umma_f16(tmem_base + b * T::kKeys, smem_desc_sw128(q_addr + blk * kRowBlock + i * 32u),
+                                 smem_desc_sw128(k_addr + blk * T::kBlock + i * 32u), T::kIdescS, (blk | i) != 0u ? 1u : 0u);
                 umma_commit(&k_empty[ks]);
                 umma_commit(&s_full[b]);
                 if (++ks == p.key_stages) ks = 0, kph ^= 1u;
@@ -191,10 +206,15 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
                 tc_fence_after();
                 const uint32_t v_addr = smem_u32(v_smem + vs * value_bytes);
 #pragma unroll
-                for (uint32_t i = 0; i < 4u; ++i) {  // 16 keys a step
-                    const uint64_t vdesc = smem_desc_sw128_mn(v_addr + i * 2048u, kKeyBlock);
-                    umma_f16(tmem_base + kOutColumn, smem_desc_sw128(hi_addr + i * 32u), vdesc, idesc_pv, (t | i) != 0u ? 1u : 0u);
-                    umma_f16(tmem_base + kOutColumn, smem_desc_sw128(lo_addr + i * 32u), vdesc, idesc_pv, 1u);
+                for (uint32_t i = 0; i < T::kKeys / 16u; ++i) {
+                    const uint64_t vdesc = smem_desc_sw128_mn(v_addr + i * 2048u, T::kBlock);
+                    if constexpr (PAGES == 1u) {
+                        umma_f16(tmem_base + T::kOutColumn, smem_desc_sw128(hi_addr + i * 32u), vdesc, idesc_pv, (t | i) != 0u ? 1u : 0u);
+                        umma_f16(tmem_base + T::kOutColumn, smem_desc_sw128(lo_addr + i * 32u), vdesc, idesc_pv, 1u);
+                    } else {
+                        umma_f16_ts(tmem_base + T::kOutColumn, tmem_base + T::kPColumn + 8u * i, vdesc, idesc_pv, (t | i) != 0u ? 1u : 0u);
+                        umma_f16_ts(tmem_base + T::kOutColumn, tmem_base + T::kPColumn + 64u + 8u * i, vdesc, idesc_pv, 1u);
+                    }
                 }
                 umma_commit(&v_empty[vs]);
                 umma_commit(p_free);
@@ -208,30 +228,31 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         const uint32_t sub = warp & 3u, half = warp >> 2;
         const uint32_t r = 32u * sub + lane, row = row0 + r;
         const uint32_t pos = p.first_pos + min(row, p.m - 1u);  // last key this row may see
-        const uint32_t lanes = (32u * sub) << 16, col0 = 32u * half;
+        const uint32_t lanes = (32u * sub) << 16, col0 = 32u * PAGES * half;
         float mrow = -INFINITY;
         uint32_t g = 0;
         bool ok = true;
+        // this thread's scores of tile b, which is free from then on
+        auto fetch_scores = [&](uint32_t b, uint32_t (&v)[PAGES][32]) {
+#pragma unroll
+            for (uint32_t c = 0; c < PAGES; ++c) tmem_ld_32x32_issue(tmem_base + lanes + b * T::kKeys + col0 + 32u * c, v[c]);
+#pragma unroll
+            for (uint32_t c = 0; c < PAGES; ++c) tmem_ld_wait_32(v[c]);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[b]);
+        };
         for (uint32_t j = 0; j < steps && ok && !p.one_pass; ++j, ++g) {
             const uint32_t b = g & 1u;
             if (!(ok = mbar_wait_bounded(&s_full[b], (g >> 1) & 1u, abort_flag))) break;
             tc_fence_after();
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + lanes + b * kKeys + col0, v);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s_free[b]);
-            const uint32_t key0 = (step0 + j) * kKeys + col0;
-            float mx = -INFINITY;
-            if (key0 + 31u <= pos) {  // the row sees the whole piece
+            uint32_t v[PAGES][32];
+            fetch_scores(b, v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(v[i]));
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (key0 + i <= pos) mx = fmaxf(mx, __uint_as_float(v[i]));
+            for (uint32_t c = 0; c < PAGES; ++c) {
+                hide_keys(v[c], (step0 + j) * T::kKeys + col0 + 32u * c, pos);
+                mrow = fmaxf(mrow, largest(v[c]) * p.scale_log2);  // the scale is positive: it commutes with the maximum
             }
-            mrow = fmaxf(mrow, mx * p.scale_log2);  // the scale is positive: it commutes with the maximum
         }
         if (p.one_pass) {
             mrow = p.bound_log2 * fabsf(query_temperature(pos, p.temp_coef, p.temp_every));
@@ -247,46 +268,45 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
                 named_bar_sync(1, kSoftmaxWarps * 32u);  // everybody has read: the words are free for the row sums
             }
         }
-        float l = 0.0f;
+        float2 sums[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
         uint8_t *p_hi = p_smem + r * 128u, *p_lo = p_hi + kRowBlock;
         for (uint32_t j = 0; j < steps && ok; ++j, ++g) {
             const uint32_t b = g & 1u;
             if (!(ok = mbar_wait_bounded(&s_full[b], (g >> 1) & 1u, abort_flag))) break;
             tc_fence_after();
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + lanes + b * kKeys + col0, v);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s_free[b]);
-            uint32_t hi[16], lo[16];
-            const uint32_t key0 = (step0 + j) * kKeys + col0;
-            const bool whole = key0 + 31u <= pos;
+            uint32_t v[PAGES][32], hi[PAGES][16], lo[PAGES][16];
+            fetch_scores(b, v);
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                // exp2 of a non-positive argument by the hardware approximation: two units of an f32's last place
-                float e0 = ex2_approx(fmaf(__uint_as_float(v[i]), p.scale_log2, -mrow));
-                float e1 = ex2_approx(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -mrow));
-                if (!whole) {
-                    if (key0 + i > pos) e0 = 0.0f;
-                    if (key0 + i + 1 > pos) e1 = 0.0f;
+            for (uint32_t c = 0; c < PAGES; ++c) {
+                hide_keys(v[c], (step0 + j) * T::kKeys + col0 + 32u * c, pos);
+                probabilities(v[c], p.scale_log2, mrow, sums, hi[c], lo[c]);
+            }
+            // the previous step's second product must have read P before it is overwritten; the warp goes on as one
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(p_free, (j & 1u) ^ 1u, abort_flag));
+            if (!ok) break;
+            if constexpr (PAGES == 1u) {
+                // 32 keys = four 16-byte chunks of the row's 128-byte line
+#pragma unroll
+                for (uint32_t q = 0; q < 4u; ++q) {
+                    const uint32_t at = ((half * 4u + q) ^ (r & 7u)) << 4;
+                    *reinterpret_cast<uint4 *>(p_hi + at) = make_uint4(hi[0][4 * q], hi[0][4 * q + 1], hi[0][4 * q + 2], hi[0][4 * q + 3]);
+                    *reinterpret_cast<uint4 *>(p_lo + at) = make_uint4(lo[0][4 * q], lo[0][4 * q + 1], lo[0][4 * q + 2], lo[0][4 * q + 3]);
                 }
-                l += e0;
-                l += e1;
-                split_bf16x2(e0, e1, hi[i >> 1], lo[i >> 1]);
-            }
-            // the previous step's second product must have read P before it is overwritten
-            if (!(ok = mbar_wait_bounded(p_free, (j & 1u) ^ 1u, abort_flag))) break;
-            // 32 keys = four 16-byte chunks of the row's 128-byte line
+                proxy_fence_async();  // the tensor core reads shared memory through the async proxy
+            } else {
+                tc_fence_after();
 #pragma unroll
-            for (uint32_t q = 0; q < 4u; ++q) {
-                const uint32_t at = ((half * 4u + q) ^ (r & 7u)) << 4;
-                *reinterpret_cast<uint4 *>(p_hi + at) = make_uint4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
-                *reinterpret_cast<uint4 *>(p_lo + at) = make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
+                for (uint32_t c = 0; c < PAGES; ++c) {  // 32 keys = 16 columns of pairs
+                    tmem_st_32x16(tmem_base + lanes + T::kPColumn + half * 32u + c * 16u, hi[c]);
+                    tmem_st_32x16(tmem_base + lanes + T::kPColumn + 64u + half * 32u + c * 16u, lo[c]);
+                }
+                tmem_st_wait();
+                tc_fence_before();
             }
-            proxy_fence_async();  // the tensor core reads shared memory through the async proxy
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full);
         }
+        float l = (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
         if constexpr (!SPLIT) {
             exchange[half * 128u + r] = l;
             named_bar_sync(1, kSoftmaxWarps * 32u);
@@ -301,7 +321,7 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         uint16_t *dst = p.out + ((size_t)row * p.heads + head) * vb * 64u + half * vb * 32u;
         for (uint32_t c = 0; c < vb; ++c) {
             uint32_t v[32], packed[16];
-            tmem_ld_32x32(tmem_base + lanes + kOutColumn + half * vb * 32u + c * 32u, v);
+            tmem_ld_32x32(tmem_base + lanes + T::kOutColumn + half * vb * 32u + c * 32u, v);
             if constexpr (SPLIT) {
                 if (!steps)
 #pragma unroll
@@ -349,11 +369,13 @@ attend_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 
 constexpr uint32_t kSmemLimit = 227u * 1024u;
 
-uint32_t stages_for(uint32_t key_blocks, uint32_t value_blocks) {
+uint32_t stages_for(uint32_t pages, uint32_t key_blocks, uint32_t value_blocks) {
     for (uint32_t k = kMaxKeyStages; k >= 2u; --k)
-        if (tc_smem_bytes(key_blocks, value_blocks, k) <= kSmemLimit) return k;
+        if (tc_smem_bytes(pages, key_blocks, value_blocks, k) <= kSmemLimit) return k;
     return 0;
 }
+// Steps of two pages where tensor memory has room for P beside O and shared memory for two stages of keys: half the hand-offs.
+uint32_t pages_for(uint32_t key_blocks, uint32_t value_blocks) { return value_blocks <= 2u && stages_for(2u, key_blocks, value_blocks) ? 2u : 1u; }
 
 // Twice the bound is how far below it a score can lie; exp2 of that must stay well inside f32 and bf16.
 constexpr float kMostBelowBound = 100.0f;
@@ -362,7 +384,7 @@ constexpr float kMostBelowBound = 100.0f;
 
 bool attend_tc_supports(uint32_t key_blocks, uint32_t value_blocks) {
     return key_blocks && value_blocks && key_blocks <= kMaxBlocks && value_blocks <= kMaxBlocks &&
-           stages_for(key_blocks, value_blocks) != 0 && encode_tiled() != nullptr;
+           stages_for(1u, key_blocks, value_blocks) != 0 && encode_tiled() != nullptr;
 }
 
 stark_b200_status attend_tc_launch(const AttendTcArgs &a, cudaStream_t stream) {
@@ -384,9 +406,9 @@ stark_b200_status attend_tc_launch(const AttendTcArgs &a, cudaStream_t stream) {
     };
     const AttendTile &shared = a.shared_blocks ? a.shared : a.keys;
     if (!make(&q_map, a.queries, (uint64_t)a.heads * key_blocks * 64u, a.m, a.ld_q, 128u) ||
-        !make(&k_map, a.keys.base, a.keys.columns, a.keys.rows, a.keys.ld, kKeys) ||
-        !make(&v_map, a.values.base, a.values.columns, a.values.rows, a.values.ld, kKeys) ||
-        !make(&shared_map, shared.base, shared.columns, shared.rows, shared.ld, kKeys))
+        !make(&k_map, a.keys.base, a.keys.columns, a.keys.rows, a.keys.ld, kPageTokens) ||
+        !make(&v_map, a.values.base, a.values.columns, a.values.rows, a.values.ld, kPageTokens) ||
+        !make(&shared_map, shared.base, shared.columns, shared.rows, shared.ld, kPageTokens))
         return STARK_B200_DEVICE_FAILURE;
     AttendTcParams p{};
     p.out = a.out;
@@ -396,7 +418,8 @@ stark_b200_status attend_tc_launch(const AttendTcArgs &a, cudaStream_t stream) {
     p.key_first = a.keys.first, p.key_stride = a.keys.stride;
     p.value_first = a.values.first, p.value_stride = a.values.stride;
     p.shared_first = a.shared.first;
-    p.key_stages = stages_for(key_blocks, a.value_blocks);
+    const uint32_t pages = pages_for(key_blocks, a.value_blocks);
+    p.key_stages = stages_for(pages, key_blocks, a.value_blocks);
     p.scale_log2 = a.scale * kLog2e;
     if (a.dim_bound > 0.0f) {
         // the temperature moves one way with the position: its largest size is at the first or the last one
@@ -407,13 +430,13 @@ stark_b200_status attend_tc_launch(const AttendTcArgs &a, cudaStream_t stream) {
         p.temp_coef = a.temp_coef, p.temp_every = a.temp_every;
     }
     p.error_word = a.error_word;
-    // two steps a CTA at least: they are half as long as those the split was measured with
-    const uint32_t split = thin_split(a.heads * ((a.m + 127u) / 128u), ((a.first_pos + a.m - 1u) / kKeys + 1u) / 2u);
-    const auto kernel = split > 1u ? attend_tc_kernel<true> : attend_tc_kernel<false>;
-    static SmemOptIn once[2];
-    if (stark_b200_status st = ensure_dynamic_smem(kernel, (int)kSmemLimit, once[split > 1u])) return st;
+    const uint32_t split = thin_split(a.heads * ((a.m + 127u) / 128u), ((a.first_pos + a.m - 1u) / kPageTokens + 1u) / 2u);
+    const auto kernel = pages == 2u ? (split > 1u ? attend_tc_kernel<true, 2u> : attend_tc_kernel<false, 2u>)
+                                    : (split > 1u ? attend_tc_kernel<true, 1u> : attend_tc_kernel<false, 1u>);
+    static SmemOptIn once[2][2];
+    if (stark_b200_status st = ensure_dynamic_smem(kernel, (int)kSmemLimit, once[pages - 1u][split > 1u])) return st;
     return thin_launch(kernel, dim3(a.heads, (a.m + 127u) / 128u, split), kThreads,
-                       tc_smem_bytes(key_blocks, a.value_blocks, p.key_stages), stream, q_map, k_map, v_map, shared_map, p);
+                       tc_smem_bytes(pages, key_blocks, a.value_blocks, p.key_stages), stream, q_map, k_map, v_map, shared_map, p);
 }
 
 bool latent_prefill_tc_supports(const LatentShape &s) { return attend_tc_supports(s.q_head() / 64u, s.vdim_p / 64u); }

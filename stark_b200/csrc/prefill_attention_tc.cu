@@ -33,6 +33,7 @@
 #include "context.cuh"
 #include "device_math.cuh"
 #include "prefill.cuh"
+#include "softmax_tc.cuh"
 #include "tc05.cuh"
 #include "thin_tile.cuh"
 #include "tunables.cuh"
@@ -56,26 +57,6 @@ constexpr uint32_t kPColumn = 384;
 constexpr uint32_t kIdescS = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t kIdescPV = kIdescS | (1u << 16);
 
-__device__ inline float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// Two f32 operations in one instruction, each rounded as the single one.
-__device__ inline float2 fma_pair(float2 a, float2 b, float2 c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(d)
-        : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)), "l"(*reinterpret_cast<uint64_t *>(&c)));
-    return *reinterpret_cast<float2 *>(&d);
-}
-__device__ inline float2 add_pair(float2 a, float2 b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t *>(&a)), "l"(*reinterpret_cast<uint64_t *>(&b)));
-    return *reinterpret_cast<float2 *>(&d);
-}
-
 // A bound (in powers of two) up to which it may stand in for a row's maximum: probabilities then lie above 2^-96, a row's largest too,
 // so that every one that counts beside it is a normal f32 -- the same relative precision as behind the maximum itself.
 constexpr float kMostBound = 48.0f;
@@ -89,14 +70,6 @@ struct TcAttnParams {
     uint32_t *error_word;
     uint32_t stop_after;  // 0 whole kernel; 1 set-up and tensor memory only; 2 pass 1 only (no MN-major operand)
 };
-
-// Scores of keys past `pos` become -inf: probabilities of exactly zero.  Only steps on the diagonal have any; the others pay one branch.
-__device__ __forceinline__ void hide_keys(uint32_t (&v)[32], uint32_t key0, uint32_t pos) {
-    if (key0 + 31u <= pos) return;
-#pragma unroll
-    for (uint32_t i = 0; i < 32u; ++i)
-        if (key0 + i > pos) v[i] = 0xff800000u;
-}
 
 constexpr uint32_t kPartPitch = 128u + 4u;  // floats between the rows of a CTA's share of O, in place of the K and V stages
 
@@ -291,10 +264,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             for (uint32_t c = 0; c < 2u; ++c) {
                 tmem_ld_wait_32(v[c]);
                 hide_keys(v[c], (step0 + j) * 128u + col0 + 32u * c, pos);
-                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains
-#pragma unroll
-                for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[c][i]));
-                mrow = fmaxf(mrow, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);  // the scale is positive: it commutes with the maximum
+                mrow = fmaxf(mrow, largest(v[c]) * p.scale_log2);  // the scale is positive: it commutes with the maximum
             }
             tc_fence_before();
             __syncwarp();
@@ -317,7 +287,6 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
         float l = 0.0f;
         float2 sums[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(-mrow, -mrow), minus1 = make_float2(-1.0f, -1.0f);
         if (passes == 2u) {
             for (uint32_t j = 0; j < steps && ok; ++j, ++g) {
                 const uint32_t b = g & 1u;
@@ -334,18 +303,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
 #pragma unroll
                 for (uint32_t c = 0; c < 2u; ++c) {
                     hide_keys(v[c], (step0 + j) * 128u + col0 + 32u * c, pos);
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        // exp2 of a non-positive argument: the hardware approximation is good to two units of an f32's
-                        // last place, far inside what the bf16 pair keeps
-                        const float2 x = fma_pair(make_float2(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), scale2, shift2);
-                        const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-                        sums[i >> 1 & 1] = add_pair(sums[i >> 1 & 1], e);
-                        const uint32_t h = f32x2_to_bf16x2(e.x, e.y);  // hi + lo: two roundings to nearest
-                        const float2 rest = fma_pair(make_float2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus1, e);
-                        hi[c][i >> 1] = h;
-                        lo[c][i >> 1] = f32x2_to_bf16x2(rest.x, rest.y);
-                    }
+                    probabilities(v[c], p.scale_log2, mrow, sums, hi[c], lo[c]);
                 }
                 // the previous step's second product must have read P before it is overwritten; the warp goes on as one
                 ok = __all_sync(0xffffffffu, mbar_wait_bounded(p_free, (j & 1u) ^ 1u, abort_flag));
