@@ -121,6 +121,8 @@ __device__ __forceinline__ void pair_gemm(const CUtensorMap &x_map, const CUtens
     pair_sync();  // the other CTA's barriers exist
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_launch_dependents();  // behind the allocation: what starts now cannot take tensor memory from a CTA that waits for it
+    pdl_wait();  // rows, weights unpacked for this launch and the residual come from the launches before
 
     // row tiles are the fast index: the pairs then share few tiles of weights, which stream from memory once, while the rows stay in L2
     if (warp == 0) {
@@ -211,13 +213,15 @@ inline stark_b200_status pair_launch(Kernel kernel, uint32_t out_cols, uint32_t 
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = kPairSmem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     SB_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
     return STARK_B200_OK;
 }

@@ -36,6 +36,7 @@ const Entry kEntries[] = {
     {"prefill_attn_warps", "STARK_B200_PREFILL_ATTN_WARPS", &Tunables::prefill_attn_warps, 4u, 4u, 8u},
     {"gemm_half_tiles", "STARK_B200_GEMM_HALF_TILES", &Tunables::gemm_half_tiles, 1u, 0u, 2u},
     {"gemm_unpack", "STARK_B200_GEMM_UNPACK", &Tunables::gemm_unpack, 1u, 0u, 2u},
+    {"gemm_pairs", "STARK_B200_GEMM_PAIRS", &Tunables::gemm_pairs, 1u, 0u, 2u},
     {"gemm_thin", "STARK_B200_GEMM_THIN", &Tunables::gemm_thin, 1u, 0u, 136u},
     {"latent_spans", "STARK_B200_LATENT_SPANS", &Tunables::latent_spans, 0u, 0u, 64u},
     {"latent_cluster", "STARK_B200_LATENT_CLUSTER", &Tunables::latent_cluster, 4u, 1u, 8u},

@@ -27,6 +27,7 @@ struct Tunables {
     uint32_t prefill_attn_warps;  // STARK_B200_PREFILL_ATTN_WARPS warps of a prompt pass's attention CTA (4 or 8): rows that share a key / value tile
     uint32_t gemm_half_tiles;     // STARK_B200_GEMM_HALF_TILES  128-row tiles in the prompt contraction: 0 never, 1 where 256-row tiles leave SMs idle, 2 always
     uint32_t gemm_unpack;         // STARK_B200_GEMM_UNPACK      weights of a prompt contraction unpacked to bf16 rows once a pass: 0 never, 1 by estimated time, 2 always
+    uint32_t gemm_pairs;          // STARK_B200_GEMM_PAIRS       256-row tiles of a bf16 prompt contraction on pairs of SMs: 0 never, 1 where they fill the SMs about as well as 128-row tiles, 2 always
     uint32_t gemm_thin;           // STARK_B200_GEMM_THIN        tiles of a prompt contraction with few row tiles: 0 the 256-feature ones, 1 by estimated time, 64 or 128 plus a split of K (1, 2, 4, 8) that tile
     uint32_t tp_rows_push;        // STARK_B200_TP_ROWS_PUSH     a prompt pass's contractions store their tiles to the other ranks themselves: 1 always, 2 between two ranks only, 0 never (a copy kernel after each)
     uint32_t rows_attention;      // STARK_B200_ROWS_ATTENTION   1: a handful of rows attend in the keys-as-rows form, 0: in 16-row tiles

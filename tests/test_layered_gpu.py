@@ -352,3 +352,23 @@ def test_invalid_requests_are_refused_on_the_host():
     m.reset()
     assert m.position == 0
     m.close()
+
+
+@pytest.mark.parametrize("rows", [17, 257, 700])
+def test_tiles_on_pairs_of_sms_leave_the_same_bits(rows):
+    """256-row tiles of the bf16 contraction on pairs of SMs against the narrow and the 128-row ones a CTA: stored, gated and f32 outputs,
+    rows and columns past the last whole tile, fewer steps than stages."""
+    from stark_b200 import _lib
+    from tests import pomelix_models as P
+    tune = lambda name, value: _lib.check(_lib.load().stark_b200_set_tunable(name, value), "set_tunable")  # noqa: E731
+    for models, root in ((L, L.model([L.layer(), L.layer()], width=328, vocab=600)), (P, P.model([P.layer(), P.layer()], width=328, vocab=600))):
+        w, ids, got = models.weights(root), models.tokens(root, rows), []
+        try:
+            tune(b"gemm_thin", 0)
+            for pairs in (0, 2):
+                tune(b"gemm_pairs", pairs)
+                got.append(run(root, w, ids, "bfloat16"))
+        finally:
+            tune(b"gemm_thin", 1)
+            tune(b"gemm_pairs", 1)
+        assert np.array_equal(got[0], got[1])
