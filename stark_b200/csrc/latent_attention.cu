@@ -5,7 +5,7 @@
 //   latent_query    per head and 64 latent columns: W_uk^T q, the rotated query part, both times scale * log2(e); one
 //                   more CTA per row norms the new latent, rotates the new key part and appends the cache row
 //   latent_attend   per span of the cached rows and group of heads: f32 scores, running softmax, weighted latents
-//   latent_value    per head and 64 output values: merge of the spans, then W_uv
+//   latent_value    per head and 32 output values: merge of the spans, then W_uv
 // Angles, norms, scores and softmax are f32.  A row of a pass attends to the rows up to its own position.
 #include "layered.cuh"
 #include "layered_math.cuh"
@@ -122,24 +122,42 @@ __global__ void __launch_bounds__(kQueryThreads) latent_query_kernel(const Laten
     }
 }
 
-// blockIdx.x: (head, 64 output values), blockIdx.y: row
+// blockIdx.x: (head, 32 output values), blockIdx.y: row.
+// Bound by its chain of trips to memory, so there is one behind the wait: the weights of this warp's rows up to rank 512 come ahead of
+// it, and the spans' partials beside their statistics.  64 values a CTA, half of the weights and all partials behind other trips: 17
+// tokens of guvulorn-8b behind 4 000 rows 61.1 -> 58.2 ms with this, 32 values and one trip (4.7 us a layer).
+constexpr uint32_t kValueRows = 4, kValueTile = 8u * kValueRows, kAhead = 2, kBatch = 8;
 template <typename O>
 __global__ void __launch_bounds__(256) latent_value_kernel(const LatentArgs a) {
     extern __shared__ __align__(16) float o[];  // [rank_p], then the pieces of the merge
     __shared__ float weight[kMaxSplits];
     const LatentShape &s = a.s;
-    const uint32_t blocks = s.vdim_p / 64u, head = blockIdx.x / blocks, piece = blockIdx.x % blocks, row = blockIdx.y;
+    const uint32_t blocks = s.vdim_p / kValueTile, head = blockIdx.x / blocks, piece = blockIdx.x % blocks, row = blockIdx.y;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint16_t *uv = a.uk_uv.data + ((size_t)s.heads * s.dim_p + (size_t)head * s.vdim_p + piece * 64u + warp * 8u) * s.rank_p;
-    // the first 256 columns of this warp's eight rows: weights do not depend on the previous kernel
-    uint4 w[8];
+    const uint32_t value0 = piece * kValueTile + warp * kValueRows;
+    const uint16_t *uv = a.uk_uv.data + ((size_t)s.heads * s.dim_p + (size_t)head * s.vdim_p + value0) * s.rank_p;
+    auto weights = [&](uint32_t j, uint32_t c) { return c < s.rank_p ? ldg_nc_v4(uv + (size_t)j * s.rank_p + c) : make_uint4(0u, 0u, 0u, 0u); };
+    uint4 w[kAhead][kValueRows];
 #pragma unroll
-    for (uint32_t j = 0; j < 8u; ++j)
-        w[j] = lane * 8u < s.rank_p ? ldg_nc_v4(uv + (size_t)j * s.rank_p + lane * 8u) : make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t i = 0; i < kAhead; ++i)
+#pragma unroll
+        for (uint32_t j = 0; j < kValueRows; ++j) w[i][j] = weights(j, i * 256u + lane * 8u);
     pdl_launch_dependents();
     pdl_wait();
     const float *part = partial_of(a, row, head, 0);
     const uint32_t pitch = s.rank_p + 4u;
+    // four columns a thread; where the latent is narrow several threads share the spans of the same four
+    const uint32_t quads = s.rank_p / 4u, shares = quads >= 256u ? 1u : 256u / quads;
+    float4 x[kBatch];
+    auto fetch = [&](uint32_t t, uint32_t k0) {
+#pragma unroll
+        for (uint32_t i = 0; i < kBatch; ++i) {
+            const uint32_t k = k0 + i * shares;
+            x[i] = t < quads * shares && k < a.splits ? *reinterpret_cast<const float4 *>(part + (size_t)k * pitch + 4u + t % quads * 4u)
+                                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    fetch(threadIdx.x, threadIdx.x / quads);
     // every warp forms the spans' weights exp2(m - max) / sum for itself; the first one leaves them for the columns
     {
         float m[2], l[2], top = -INFINITY, sum = 0.0f;
@@ -160,17 +178,19 @@ __global__ void __launch_bounds__(256) latent_value_kernel(const LatentArgs a) {
         if (warp == 0u) weight[lane] = m[0] * inv, weight[lane + 32u] = m[1] * inv;
     }
     __syncthreads();
-    // four columns a thread; where the latent is narrow several threads share the spans of the same four
-    const uint32_t quads = s.rank_p / 4u, shares = quads >= 256u ? 1u : 256u / quads;
     float4 *pieces = reinterpret_cast<float4 *>(o + s.rank_p);  // [shares][quads]
     for (uint32_t t = threadIdx.x; t < quads * shares; t += 256u) {
-        const uint32_t quad = t % quads, share = t / quads;
+        const uint32_t share = t / quads;
+        if (t != threadIdx.x) fetch(t, share);
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 8
-        for (uint32_t k = share; k < a.splits; k += shares) {
-            const float4 x = *reinterpret_cast<const float4 *>(part + (size_t)k * pitch + 4u + quad * 4u);
-            const float c = weight[k];
-            v.x = fmaf(c, x.x, v.x), v.y = fmaf(c, x.y, v.y), v.z = fmaf(c, x.z, v.z), v.w = fmaf(c, x.w, v.w);
+        for (uint32_t k0 = share; k0 < a.splits; k0 += kBatch * shares) {
+            if (k0 != share) fetch(t, k0);
+#pragma unroll
+            for (uint32_t i = 0; i < kBatch; ++i) {
+                if (k0 + i * shares >= a.splits) break;
+                const float c = weight[k0 + i * shares];
+                v.x = fmaf(c, x[i].x, v.x), v.y = fmaf(c, x[i].y, v.y), v.z = fmaf(c, x[i].z, v.z), v.w = fmaf(c, x[i].w, v.w);
+            }
         }
         pieces[t] = v;
     }
@@ -178,31 +198,40 @@ __global__ void __launch_bounds__(256) latent_value_kernel(const LatentArgs a) {
     for (uint32_t quad = threadIdx.x; quad < quads; quad += 256u) {
         float4 v = pieces[quad];
         for (uint32_t k = 1; k < shares; ++k) {
-            const float4 x = pieces[k * quads + quad];
-            v.x += x.x, v.y += x.y, v.z += x.z, v.w += x.w;
+            const float4 y = pieces[k * quads + quad];
+            v.x += y.x, v.y += y.y, v.z += y.z, v.w += y.w;
         }
         reinterpret_cast<float4 *>(o)[quad] = v;
     }
     __syncthreads();
-    float acc[8] = {};
-    for (uint32_t c = lane * 8u; c < s.rank_p; c += 256u) {
-        const float4 x = *reinterpret_cast<const float4 *>(o + c), y = *reinterpret_cast<const float4 *>(o + c + 4u);
+    float acc[kValueRows] = {};
+    auto columns = [&](uint32_t c, const uint4 (&now)[kValueRows]) {
+        const float4 l = *reinterpret_cast<const float4 *>(o + c), r = *reinterpret_cast<const float4 *>(o + c + 4u);
 #pragma unroll
-        for (uint32_t j = 0; j < 8u; ++j) {
-            const uint4 v = c < 256u ? w[j] : ldg_nc_v4(uv + (size_t)j * s.rank_p + c);
-            acc[j] = fmaf(__uint_as_float(v.x << 16), x.x, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.x & 0xffff0000u), x.y, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.y << 16), x.z, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.y & 0xffff0000u), x.w, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.z << 16), y.x, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.z & 0xffff0000u), y.y, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.w << 16), y.z, acc[j]);
-            acc[j] = fmaf(__uint_as_float(v.w & 0xffff0000u), y.w, acc[j]);
+        for (uint32_t j = 0; j < kValueRows; ++j) {
+            const uint4 v = now[j];
+            acc[j] = fmaf(__uint_as_float(v.x << 16), l.x, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.x & 0xffff0000u), l.y, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.y << 16), l.z, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.y & 0xffff0000u), l.w, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.z << 16), r.x, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.z & 0xffff0000u), r.y, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.w << 16), r.z, acc[j]);
+            acc[j] = fmaf(__uint_as_float(v.w & 0xffff0000u), r.w, acc[j]);
         }
-    }
-    O *dst = reinterpret_cast<O *>(a.out) + ((size_t)row * s.heads + head) * s.vdim_p + piece * 64u + warp * 8u;
+    };
 #pragma unroll
-    for (uint32_t j = 0; j < 8u; ++j) {
+    for (uint32_t i = 0; i < kAhead; ++i)
+        if (i * 256u + lane * 8u < s.rank_p) columns(i * 256u + lane * 8u, w[i]);
+    for (uint32_t c = kAhead * 256u + lane * 8u; c < s.rank_p; c += 256u) {
+        uint4 now[kValueRows];
+#pragma unroll
+        for (uint32_t j = 0; j < kValueRows; ++j) now[j] = weights(j, c);
+        columns(c, now);
+    }
+    O *dst = reinterpret_cast<O *>(a.out) + ((size_t)row * s.heads + head) * s.vdim_p + value0;
+#pragma unroll
+    for (uint32_t j = 0; j < kValueRows; ++j) {
         const float v = warp_sum(acc[j]);
         if (lane == 0) store_value(dst + j, v);
     }
@@ -273,7 +302,7 @@ stark_b200_status latent_value_launch(const LatentArgs &a, cudaStream_t stream) 
     if (stark_b200_status st = check_args(a)) return st;
     if (!a.partials || !a.out) return STARK_B200_INVALID_ARGUMENT;
     auto kernel = a.out_b16 ? latent_value_kernel<uint16_t> : latent_value_kernel<float>;
-    return launch_chained(kernel, dim3(a.s.heads * (a.s.vdim_p / 64u), a.m), dim3(256),
+    return launch_chained(kernel, dim3(a.s.heads * (a.s.vdim_p / kValueTile), a.m), dim3(256),
                           a.s.rank_p * 4u + std::max(a.s.rank_p * 4u, 4096u), a.pdl, stream, a);
 }
 

@@ -68,6 +68,16 @@ def test_attention_alone(dtype, mix, scaling):
 
 
 @BOTH
+@pytest.mark.parametrize("rank,vdim", [(33, 200), (260, 65), (700, 40)])
+def test_values_of_narrow_and_wide_latents(dtype, rank, vdim):
+    """The values' merge and product: spans divided among threads, one batch of spans and several, columns past the weights fetched ahead."""
+    root = L.model([L.layer(L.mixer(heads=2, dim=24, rot_dim=12, vdim=vdim, kv_rank=rank), ff=None)])
+    w = L.weights(root, seed=11)
+    ids = L.tokens(root, 140)
+    close(run(root, w, ids, dtype, [130] + [1] * 10), L.oracle(root, w).feed(ids), dtype)
+
+
+@BOTH
 @pytest.mark.parametrize("ff,limit", [(40, 0.7), (16, 3.0), (1, 1.0), (200, 0.25)])
 def test_feed_forward_alone(dtype, ff, limit):
     root = L.model([L.layer(ff=ff, limit=limit)])
