@@ -176,7 +176,7 @@ def test_column_slices(rows, columns):
     make = lambda pair: QMatrix.from_affine(w["codes"], w["scales"], w["biases"], rows, columns, pair_halves=pair)  # noqa: E731
     plain, pair = make(False), make(True) if rows % 32 == 0 else None
     rng = np.random.default_rng(rows)
-    several = {m: S.bf16_normal(rng, m * columns).reshape(m, columns) for m in (2, 5, 8)}
+    several = {m: S.bf16_normal(rng, m * columns).reshape(m, columns) for m in (2, 5, 8) if m * columns <= 8 * 8192}  # more: refused
     weight = (1.0 + 0.1 * rng.standard_normal(columns)).astype(np.float32)
     seen = []
     try:
