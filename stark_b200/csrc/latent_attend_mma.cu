@@ -286,16 +286,28 @@ latent_attend_mma_kernel(const __grid_constant__ CUtensorMap map, const AttendPa
     const uint32_t me = span_i % p.cluster, split_i = span_i / p.cluster;
     // thread = (head, quads of this CTA's columns); an empty span's weight is 0 and its latents are zeros
     const uint32_t h = tid >> 4, head = head0 + h, quads = rank / 4u;
-    float weight[kMaxCluster], top = -INFINITY, sum = 0.0f;
+    // statistics and the first columns of all spans are on their way before the first is used: one trip instead of three
+    // (17 tokens of guvulorn-8b behind 4 000 rows 58.26 -> 58.01 ms, runs 0.03 apart)
+    float weight[kMaxCluster], sums[kMaxCluster], top = -INFINITY, sum = 0.0f;
+    float4 x[kMaxCluster];
+    auto fetch_columns = [&](uint32_t q) {
+#pragma unroll
+        for (uint32_t c = 0; c < kMaxCluster; ++c)
+            x[c] = c < p.cluster && q < quads ? peer_load4(peer_smem(state + h * rank + q * 4u, c)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    const uint32_t first = me + p.cluster * (tid & 15u);
 #pragma unroll
     for (uint32_t c = 0; c < kMaxCluster; ++c) {
         weight[c] = c < p.cluster ? peer_load(peer_smem(&run_m[h], c)) : -INFINITY;
-        top = fmaxf(top, weight[c]);
+        sums[c] = c < p.cluster ? peer_load(peer_smem(&run_l[h], c)) : 0.0f;
     }
+    fetch_columns(first);
+#pragma unroll
+    for (uint32_t c = 0; c < kMaxCluster; ++c) top = fmaxf(top, weight[c]);
 #pragma unroll
     for (uint32_t c = 0; c < kMaxCluster; ++c) {
         weight[c] = weight[c] == -INFINITY ? 0.0f : exp2f(weight[c] - top);
-        if (c < p.cluster) sum = fmaf(weight[c], peer_load(peer_smem(&run_l[h], c)), sum);
+        if (c < p.cluster) sum = fmaf(weight[c], sums[c], sum);
     }
     if (head < p.heads) {
         float *dst = p.partials + (((size_t)row * p.heads + head) * p.splits + split_i) * (rank + 4u);
@@ -303,15 +315,15 @@ latent_attend_mma_kernel(const __grid_constant__ CUtensorMap map, const AttendPa
             dst[0] = top;  // -infinity: no span of the cluster had a page
             dst[1] = sum;
         }
-        for (uint32_t q = me + p.cluster * (tid & 15u); q < quads; q += 16u * p.cluster) {
+        for (uint32_t q = first; q < quads; q += 16u * p.cluster) {
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
             for (uint32_t c = 0; c < kMaxCluster; ++c) {
                 if (c >= p.cluster) break;
-                const float4 x = peer_load4(peer_smem(state + h * rank + q * 4u, c));
-                v.x = fmaf(weight[c], x.x, v.x), v.y = fmaf(weight[c], x.y, v.y);
-                v.z = fmaf(weight[c], x.z, v.z), v.w = fmaf(weight[c], x.w, v.w);
+                v.x = fmaf(weight[c], x[c].x, v.x), v.y = fmaf(weight[c], x[c].y, v.y);
+                v.z = fmaf(weight[c], x[c].z, v.z), v.w = fmaf(weight[c], x[c].w, v.w);
             }
+            fetch_columns(q + 16u * p.cluster);
             *reinterpret_cast<float4 *>(dst + 4u + q * 4u) = v;
         }
     }
